@@ -90,7 +90,7 @@ def draw(rng):
         return dict(family=family, nr=_log(rng, 9, 64), nt=_log(rng, 16, 128), N=rng.randint(2, 6),
                     precision=precision, steps=4)
     if family == "shock":
-        return dict(family=family, nx=_log(rng, 64, 512), ny=_log(rng, 4, 80), N=rng.randint(2, 5),
+        return dict(family=family, nx=_log(rng, 64, 512), ny=_log(rng, 4, 80), N=rng.randint(3, 5),
                     precision=precision, sensor=sensor, steps=10)
     if family == "kh":
         return dict(family=family, n=_log(rng, 16, 300), N=rng.randint(3, 7), precision=precision, sensor=sensor,
