@@ -106,10 +106,11 @@ static void health_check(hg_ctx* c) {
   HG_CUDA(cudaStreamSynchronize(c->stream));
   int w[2] = {0, -1};
   HG_CUDA(cudaMemcpy(w, c->d_health, sizeof(w), cudaMemcpyDeviceToHost));
-  if ((w[0] & c->health_fatal) == 0) {
+  if ((w[0] & (c->health_fatal | HEALTH_COPY)) == 0) {
     *reinterpret_cast<volatile int*>(c->h_health) = 0;
     return;
   }
+  if (w[0] & HEALTH_COPY) throw std::runtime_error("a stage kernel gave up waiting for its copies; set a new state to continue");
   std::string what;
   if (w[0] & HEALTH_NONFINITE) what += " a non-finite value";
   if (w[0] & HEALTH_DENSITY) what += std::string(what.empty() ? "" : ",") + " a non-positive density";
@@ -118,15 +119,18 @@ static void health_check(hg_ctx* c) {
                 "); set a new state to continue");
 }
 
-static int epb_of(const hg_ctx* c, int variant) {
-  return c->ns ? epb_ns_of(c->P, variant) : epb_stage(c->P, variant);
+// Tiling of the Euler stage kernel: variant 0's groups of elements are cut to variant 1's where they would
+// leave half of the SMs or more without one (fewer than two groups per SM): there a stage is one pass of
+// latency, and the smaller groups spread it over the chip.
+static int stage_variant(const hg_ctx* c, int variant) {
+  return variant || c->n_el < 2 * c->n_sm * epb_stage(c->P, 0) ? 1 : 0;
 }
-static int grid_for(const hg_ctx* c) {
-  const int epb = epb_of(c, c->tiling);
-  return (c->n_el + epb - 1) / epb;
+static int epb_of(const hg_ctx* c, int variant) {
+  return c->ns ? epb_ns_of(c->P, variant) : epb_stage(c->P, stage_variant(c, variant));
 }
 // per-CTA residual partials: room for the tiling variant with the most CTAs
 static int max_grid(const hg_ctx* c) {
+  if (!c->ns) return std::min(c->n_el, 32 * c->n_sm);
   const int epb = std::min(epb_of(c, 0), epb_of(c, 1));
   return (c->n_el + epb - 1) / epb;
 }
@@ -189,7 +193,7 @@ static void ns_dispatch(hg_ctx* c, const NSArgs<real>& a) {
   }
 template <int P, typename real>
 static void stage_dispatch(hg_ctx* c, const StageArgs<real>& a) {
-  if (c->tiling) launch_stage_PV<P, real, 1>(c, a);
+  if (stage_variant(c, c->tiling)) launch_stage_PV<P, real, 1>(c, a);
   else launch_stage_PV<P, real, 0>(c, a);
 }
 
@@ -266,7 +270,6 @@ static void run_stage(hg_ctx* c, double ca, double cb, double cc, bool first, bo
   a.side = c->d_side;
   a.side_geo = static_cast<const real*>(c->d_side_geo);
   a.vol_geo = static_cast<const real*>(c->d_vol_geo);
-  a.mats = c->d_mats;
   a.zones = c->d_zones;
   a.bq = c->d_bq;
   a.FX = static_cast<const real*>(c->d_FX);
@@ -424,6 +427,8 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
   cudaDeviceProp prop;
   HG_CUDA(cudaGetDeviceProperties(&prop, dev));
   if (prop.major < 10) throw std::runtime_error("libhorsesgpu requires an sm_100 (Blackwell) device");
+  c->device = dev;
+  c->n_sm = prop.multiProcessorCount;
   const int E = m->n_elements;
   if (E <= 0) throw std::runtime_error("mesh has no elements");
   const int N = m->N[0];
@@ -476,13 +481,11 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
   c->sensor_s0 = std::log10(1.0 / std::pow(double(N + 1), 4.0));   // modal ramp defaults
   c->sensor_kappa = 1.0;
 
-  // volume metrics
-  std::vector<double> vg(size_t(E) * NP * 5);
-  for (size_t n = 0; n < size_t(E) * NP; ++n) {
-    for (int k = 0; k < 4; ++k) vg[n * 5 + k] = m->Ja[n * 4 + k];
+  // volume metrics of node n: Ja00 Ja01 Ja10 Ja11 1/J
+  for (size_t n = 0; n < size_t(E) * NP; ++n)
     if (!(m->jac[n] > 0.0)) throw std::runtime_error("non-positive mapping jacobian");
-    vg[n * 5 + 4] = 1.0 / m->jac[n];
-  }
+  auto metric = [&](size_t n, int k) { return k < 4 ? m->Ja[n * 4 + k] : 1.0 / m->jac[n]; };
+  std::vector<double> vg;
 
   // zones
   std::vector<Zone> zones(std::max(1, n_bcs));
@@ -571,12 +574,14 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
     auto close = [](double a, double b, double scale) { return std::fabs(a - b) <= 1e-14 * scale; };
     bool aff = true;
     for (int e = 0; e < E && aff; ++e) {
-      const double* g0 = &vg[size_t(e) * NP * 5];
-      double sc = 0.0;
+      const size_t n0 = size_t(e) * NP;
+      double g0[5], sc = 0.0;
+      for (int k = 0; k < 5; ++k) g0[k] = metric(n0, k);
       for (int k = 0; k < 4; ++k) sc = std::fmax(sc, std::fabs(g0[k]));
-      for (int n = 1; n < NP && aff; ++n)
-        for (int k = 0; k < 5; ++k)
-          if (!close(g0[n * 5 + k], g0[k], k < 4 ? sc : std::fabs(g0[4]))) { aff = false; break; }
+      for (int n = 1; n < NP && aff; ++n) {
+        for (int k = 0; k < 4 && aff; ++k) aff = close(m->Ja[(n0 + n) * 4 + k], g0[k], sc);
+        if (aff && m->jac[n0 + n] != m->jac[n0]) aff = close(metric(n0 + n, 4), g0[4], std::fabs(g0[4]));
+      }
       for (int s = 0; s < 4 && aff; ++s) {
         const double* s0 = &sg[(size_t(e) * 4 + s) * P * 3];
         for (int k = 1; k < P && aff; ++k)
@@ -585,14 +590,20 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
       }
     }
     c->affine = aff;
+    // element records (vol_geo_stride, hg_stage.cuh)
+    const size_t stride = vol_geo_stride(P, aff);
+    vg.assign(size_t(E) * stride, 0.0);
+    for (int e = 0; e < E; ++e) {
+      double* r = &vg[size_t(e) * stride];
+      for (int n = 0; n < (aff ? 1 : NP); ++n)
+        for (int k = 0; k < 5; ++k) r[n * 5 + k] = metric(size_t(e) * NP + n, k);
+    }
     if (aff) {
-      std::vector<double> vg1(size_t(E) * 5), sg1(size_t(E) * 4 * 3);
-      for (int e = 0; e < E; ++e) {
-        for (int k = 0; k < 5; ++k) vg1[size_t(e) * 5 + k] = vg[size_t(e) * NP * 5 + k];
+      std::vector<double> sg1(size_t(E) * 4 * 3);
+      for (int e = 0; e < E; ++e)
         for (int s = 0; s < 4; ++s)
-          for (int q = 0; q < 3; ++q) sg1[(size_t(e) * 4 + s) * 3 + q] = sg[(size_t(e) * 4 + s) * P * 3 + q];
-      }
-      vg.swap(vg1);
+          for (int q = 0; q < 3; ++q)
+            vg[size_t(e) * stride + 8 + s * 3 + q] = sg1[(size_t(e) * 4 + s) * 3 + q] = sg[(size_t(e) * 4 + s) * P * 3 + q];
       sg.swap(sg1);
     }
   }
@@ -689,6 +700,7 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
   }
   c->h_side = side;
   HG_CUDA(cudaMemcpy(c->d_side, side.data(), side.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  c->h_mats = mats;
   HG_CUDA(cudaMemcpy(c->d_mats, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
   HG_CUDA(cudaMemcpy(c->d_zones, zones.data(), zones.size() * sizeof(Zone), cudaMemcpyHostToDevice));
   HG_CUDA(cudaMemset(c->d_resid, 0, size_t(max_grid(c)) * 4 * sizeof(double)));
@@ -998,7 +1010,7 @@ extern "C" int hg_residuals(hg_ctx* c, double out[4]) {
       return 0;
     }
     timed(c, HG_KERNEL_REDUCE,
-          [&] { residual_reduce_kernel<<<1, 256, 0, c->stream>>>(grid_for(c), c->d_resid, c->d_resid_out); });
+          [&] { residual_reduce_kernel<<<1, 256, 0, c->stream>>>(c->n_resid, c->d_resid, c->d_resid_out); });
     ++c->launches;
     HG_CUDA(cudaGetLastError());
     HG_CUDA(cudaMemcpyAsync(out, c->d_resid_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1556,7 +1568,7 @@ extern "C" int hg_get_tiling(const hg_ctx* c, int32_t out[3]) {
   const int epb = epb_of(c, c->tiling);
   out[0] = c->tiling;
   out[1] = epb;
-  out[2] = block_of(c->P, epb);
+  out[2] = c->ns ? block_of(c->P, epb) : stage_threads(c->P, stage_variant(c, c->tiling));
   return 0;
 }
 

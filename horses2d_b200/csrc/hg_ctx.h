@@ -26,12 +26,15 @@ struct hg_ctx {
   void* d_side_geo = nullptr;     // geometry in the context's precision (FP32 path: float)
   void* d_vol_geo = nullptr;
   double* d_mats = nullptr;
+  std::vector<double> h_mats;     // the nodal operators (layout of d_mats)
+  int device = 0, n_sm = 1;
   Zone* d_zones = nullptr;
   double* d_Q = nullptr;
   void* d_G = nullptr;
   void* d_T[2] = {nullptr, nullptr};
   double* d_QDot = nullptr;
-  double* d_resid = nullptr;      // per-CTA partial maxima of |QDot| of the last stage [grid][4]
+  double* d_resid = nullptr;      // per-CTA partial maxima of |QDot| of the last stage [n_resid][4]
+  int n_resid = 1;                // CTAs of that stage
   double* d_resid_out = nullptr;  // reduced maxima [4]
   double* d_elmax = nullptr;      // [n_el][4] umax, amax per element and their NaN flags
   int cur = 0;                    // which trace buffer holds the current traces
@@ -197,6 +200,7 @@ inline bool is_composite(const hg_ctx* c) { return !c->parts.empty(); }
 inline bool ns_fused(const hg_ctx* c) {
   return c->ns && c->ip && !c->is_part && !is_composite(c) && (c->av == HG_AV_NONE || c->sensor_kind != 0);
 }
+constexpr int HG_KNOWN_DEVICES = 16;   // devices whose kernel occupancy is looked up once
 constexpr int HG_MAX_PARTS = 12;
 constexpr int HG_MAX_ORDER_EULER = 12;
 constexpr int HG_MAX_ORDER_NS = 10;

@@ -3,30 +3,61 @@
 #pragma once
 #include "hg_ctx.h"
 
+#include <algorithm>
+#include <atomic>
+
+// Resident CTAs per SM of a persistent kernel with `smem` bytes of dynamic shared memory, after allowing it
+// that much; looked up once per kernel and device.
+template <typename K>
+static int resident_ctas(const hg_ctx* c, std::atomic<int>* known, K kernel, int threads, size_t smem) {
+  std::atomic<int>* slot = c->device < HG_KNOWN_DEVICES ? &known[c->device] : nullptr;
+  int n = slot ? slot->load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  max_carveout(kernel);
+  HG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
+  if (n < 1) throw std::runtime_error("stage kernel does not fit on this device");
+  if (slot) slot->store(n, std::memory_order_relaxed);
+  return n;
+}
+
+template <int P, typename real>
+static StageOps<P, real> stage_ops(const hg_ctx* c) {
+  StageOps<P, real> o;
+  const double* m = c->h_mats.data();
+  for (int k = 0; k < P * P; ++k) o.hatD[k] = real(m[k]);
+  m += P * P;
+  for (int k = 0; k < P; ++k) {
+    o.lb0[k] = real(m[k]);
+    o.lb1[k] = real(m[P + k]);
+    o.lbw0[k] = real(m[2 * P + k]);
+    o.lbw1[k] = real(m[3 * P + k]);
+  }
+  return o;
+}
+
+template <int P, typename real, int V, bool AFFINE, bool LGL>
+static void launch_stage_PAL(hg_ctx* c, const StageArgs<real>& a) {
+  using Tl = StageTiles<P, V, real, AFFINE, LGL>;
+  static std::atomic<int> known[HG_KNOWN_DEVICES];
+  const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
+  const int most = c->n_sm * std::min(32, resident_ctas(c, known, stage_kernel<P, V, real, AFFINE, LGL>, Tl::T, sizeof(Tl)));
+  // every CTA takes the same number of groups but the last ones: no more CTAs than that needs
+  const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
+  if (a.resid) c->n_resid = grid;
+  const StageOps<P, real> op = stage_ops<P, real>(c);
+  timed(c, HG_KERNEL_STAGE, [&] { stage_kernel<P, V, real, AFFINE, LGL><<<grid, Tl::T, sizeof(Tl), c->stream>>>(a, op); });
+  ++c->launches;
+}
+
 template <int P, typename real, int V>
 void launch_stage_PV(hg_ctx* c, const StageArgs<real>& a) {
-  constexpr int EPB = epb_stage(P, V);
-  constexpr int BLK = block_of(P, EPB);
-  const int grid = (a.n_el + EPB - 1) / EPB;
-  static bool attr = false;
-  if (!attr) {
-    max_carveout(stage_kernel<P, EPB, real, true, false>);
-    max_carveout(stage_kernel<P, EPB, real, false, false>);
-    max_carveout(stage_kernel<P, EPB, real, true, true>);
-    max_carveout(stage_kernel<P, EPB, real, false, true>);
-    attr = true;
-  }
   const bool lgl = c->node_type == HG_NODES_LGL;
-  timed(c, HG_KERNEL_STAGE, [&] {
-    if (c->affine) {
-      if (lgl) stage_kernel<P, EPB, real, true, true><<<grid, BLK, 0, c->stream>>>(a);
-      else stage_kernel<P, EPB, real, true, false><<<grid, BLK, 0, c->stream>>>(a);
-    } else {
-      if (lgl) stage_kernel<P, EPB, real, false, true><<<grid, BLK, 0, c->stream>>>(a);
-      else stage_kernel<P, EPB, real, false, false><<<grid, BLK, 0, c->stream>>>(a);
-    }
-  });
-  ++c->launches;
+  if (c->affine) {
+    if (lgl) launch_stage_PAL<P, real, V, true, true>(c, a); else launch_stage_PAL<P, real, V, true, false>(c, a);
+  } else {
+    if (lgl) launch_stage_PAL<P, real, V, false, true>(c, a); else launch_stage_PAL<P, real, V, false, false>(c, a);
+  }
 }
 
 template <int P, typename real>
@@ -35,7 +66,7 @@ void launch_trace_P(hg_ctx* c) {
   const int grid = (c->n_el + EPB - 1) / EPB;
   timed(c, HG_KERNEL_TRACE, [&] {
     trace_kernel<P, EPB, real><<<grid, block_for(P), 0, c->stream>>>(c->n_el, c->d_Q, c->d_mats,
-                                                                     static_cast<real*>(c->d_T[c->cur]));
+                                                                     static_cast<real*>(c->d_T[c->cur]), c->ns);
   });
   ++c->launches;
 }
@@ -57,6 +88,7 @@ static void launch_ns_PAI(hg_ctx* c, const NSArgs<real>& a) {
     ++c->launches;
   }
   if (a.run_stage) {
+    if (a.resid) c->n_resid = grid;
     timed(c, HG_KERNEL_STAGE,
           [&] { ns_stage_kernel<P, EPB, real, AFFINE, IP, AV><<<grid, BLK, 0, c->stream>>>(a); });
     ++c->launches;

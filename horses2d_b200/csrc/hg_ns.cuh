@@ -36,7 +36,7 @@ struct NSArgs {
   const int4* side;         // [n_el*4] {neighbour trace slot, flags, zone, per-node state row or -1}
   const real* side_geo;     // normals / dS (per node, or per side when AFFINE)
   const double* side_invh;  // [n_el*4] invh of the side's edge
-  const real* vol_geo;      // Ja00 Ja01 Ja10 Ja11 1/J (per node, or per element when AFFINE)
+  const real* vol_geo;      // element records of vol_geo_stride reals (hg_stage.cuh)
   const real* jac;          // [n_el][NP] J per node (curved meshes)
   const double* mats;       // hatD[NP] lb0 lb1 lbw0 lbw1 [P each] D[NP] dlbw0 dlbw1 [P each]
   const Zone* zones;
@@ -269,9 +269,9 @@ __device__ __forceinline__ void load_tiles(const NSArgs<real>& a, NSTiles<P, EPB
     s.Q[2][le][tid] = real(q23.x); s.Q[3][le][tid] = real(q23.y);
     if constexpr (AFFINE) {
 #pragma unroll
-      for (int k = 0; k < 5; ++k) geoE[k] = real(a.vol_geo[size_t(e) * 5 + k]);
+      for (int k = 0; k < 5; ++k) geoE[k] = a.vol_geo[size_t(e) * vol_geo_stride(P, true) + k];
     } else {
-      const real* gp = a.vol_geo + (size_t(e) * NP + tid) * 5;
+      const real* gp = a.vol_geo + size_t(e) * vol_geo_stride(P, false) + tid * 5;
 #pragma unroll
       for (int k = 0; k < 4; ++k) s.Ja[k][le][tid] = real(gp[k]);
       s.Ja[4][le][tid] = real(a.jac[size_t(e) * NP + tid]);

@@ -1,29 +1,36 @@
 // hg_stage.cuh -- the fused DGSEM stage kernel (Euler) for sm_100a.
 //
-// One launch = one Runge-Kutta stage (or one bare time derivative) over all
-// elements.  Per element (one thread per node, EPB elements per CTA):
-//   1. load Q (reference layout, 32 B per node: coalesced) and the metrics;
-//   2. Euler flux -> contravariant fluxes into shared memory
-//        (Scalar_StdVolumeGreen, Approximation/DGWeakIntegrals.f90:111-181);
-//   3. 4(N+1) face-node tasks: own trace (from shared memory) and the neighbour's
-//      trace of the previous stage (global, written by that element's previous
-//      launch), Riemann solver / boundary state, x dS
-//        (ComputeRiemannSolver_*, DGSpatialDiscretizationMethods.f90:545-1511;
-//         projections types 1-2, Mesh/QuadElement_EdgeProcedures.incf:749-1206);
-//   4. volume contraction with hatD, surface lift with lbw (Scalar_StdFace,
-//      DGWeakIntegrals.f90:183-266), division by J (computeQDot :226-233);
-//   5. low-storage RK update G = a G + b QDot, Q += c G
-//        (DGTimeIntegrator.f90:282-365), in place;
-//   6. traces of the new Q on the 4 sides for the next launch (ping-pong buffer)
-//        (interpolateSolutionToBoundaries, :1520-1574).
-// The Riemann flux of an interior face is evaluated by both of its elements with
-// identical arguments (LEFT trace, RIGHT trace, LEFT's normal), so both see the
-// same value and the face needs no separate launch or flux buffer.
+// One launch = one Runge-Kutta stage (or one bare time derivative) over all elements, in place.  CTAs
+// are persistent: each walks over groups of EPB consecutive elements, and while it works on one group
+// the inputs of its next one travel into the other half of a double buffer (state, RK register, own
+// traces, metrics and the side table of the group after it as bulk copies on an mbarrier; the
+// neighbours' traces as 16-byte asynchronous copies, because their addresses come from the side table).
+// Per group, with a barrier between the phases:
+//   A  face nodes and volume nodes as one list of items over all threads (whole warps of each kind):
+//      a face node takes its own and the neighbour's trace and solves the Riemann problem / boundary
+//      state, x dS (ComputeRiemannSolver_*, DGSpatialDiscretizationMethods.f90:545-1511; projections
+//      types 1-2, Mesh/QuadElement_EdgeProcedures.incf:749-1206); a volume node forms its contravariant
+//      fluxes (Scalar_StdVolumeGreen, Approximation/DGWeakIntegrals.f90:111-181);
+//   B  one thread per (variable, line of nodes, direction): the line's P fluxes in registers, contracted
+//      with hatD and lifted with lbw at its two ends (Scalar_StdFace, DGWeakIntegrals.f90:183-266), back
+//      in place;
+//   C  per node: division by J (computeQDot :226-233), low-storage RK update G = a G + b QDot,
+//      Q += c G (DGTimeIntegrator.f90:282-365); Gauss-Lobatto: the boundary nodes are the new traces;
+//   D  Legendre-Gauss: one thread per (variable, line): the traces of the new state at the line's ends
+//      (interpolateSolutionToBoundaries, :1520-1574) for the next launch (ping-pong buffer).
+// What bounds it: instruction issue and HBM.  One thread per node with its loads where they were used (the
+// form before) spent half of its warps' cycles on global loads and filled 62 % of the lanes of its face
+// phase; measured with 512 x 512 elements, N = 4, Gauss-Lobatto, FP64: 0.80 ms a stage then, 0.32 ms now
+// (1.17 GB of state, register and trace traffic: 3.7 TB/s); 16 x 16 elements: 20.5 -> 14.3 us a step.
+// The Riemann flux of an interior face is evaluated by both of its elements with identical arguments
+// (LEFT trace, RIGHT trace, LEFT's normal), so both see the same value and the face needs no separate
+// launch or flux buffer.
 //
-// CTAs are one-dimensional, padded to whole warps (threads past EPB*(N+1)^2 only
-// take part in barriers and reductions).  Shared tiles are variable-major
-// ([var][element][node]) so that a warp reading one row or column of a tile
-// touches consecutive words.
+// The nodal operators are kernel parameters: with the line loops unrolled their entries are constant-bank
+// operands of the multiply-adds, so a line costs P shared loads and P stores for P^2 multiply-adds (one
+// thread per node needs 2P loads for 2P multiply-adds).  Shared tiles are variable-major with rows of
+// an odd number of nodes (PO) and a variable stride VS = 4 (8 in float) modulo the bank count: lanes that
+// walk along rows, columns or (variable, line) pairs all touch different banks.
 #pragma once
 #include "hg_physics.cuh"
 #include "hg_bc.cuh"
@@ -40,8 +47,7 @@ struct StageArgs {
   int n_el;
   const int4* side;        // [n_el*4] {neighbour trace slot, flags, zone, per-node state row or -1}
   const real* side_geo;    // [n_el*4][P][3] (or [n_el*4][3] affine)  nx, ny, dS in this element's side order
-  const real* vol_geo;     // [n_el][P*P][5] (or [n_el][5] affine)  Ja00 Ja01 Ja10 Ja11 1/J
-  const double* mats;      // hatD[P*P], lb0[P], lb1[P], lbw0[P], lbw1[P]
+  const real* vol_geo;     // element records of vol_geo_stride reals (below)
   const Zone* zones;
   const double* bq;        // per-node Dirichlet states [rows][P][4] (sides whose side.w >= 0)
   const real* FX;          // exact-solver face fluxes [n_el*4][P][4] of this stage (RIEMANN_EXACT faces)
@@ -61,17 +67,31 @@ struct StageArgs {
   PhysConst pc;
 };
 
-// Elements per CTA: tiling variant 0 (default, large CTAs) and variant 1 (small CTAs: more CTAs in
-// flight on small meshes); hg_autotune times both on the resident state and keeps the faster.
-__host__ __device__ constexpr int epb_for(int P) {
-  return P == 2 ? 32 : P == 3 ? 16 : P == 4 ? 16 : P == 5 ? 8 : P == 6 ? 8 : P == 7 ? 4 : P == 8 ? 4 : P <= 11 ? 3 : 2;
-}
-__host__ __device__ constexpr int epb_small_for(int P) {
-  return P == 2 ? 8 : P == 3 ? 4 : P == 4 ? 4 : P == 5 ? 2 : P == 6 ? 2 : P == 7 ? 2 : 1;
-}
+// Metrics record of an element, a multiple of 16 bytes long in either precision.  Curved: [P*P][5] with
+// Ja00 Ja01 Ja10 Ja11 1/J per node.  Affine (AFFINE_REC reals): those five, three unused, then nx ny dS of
+// the four sides.
+constexpr int AFFINE_REC = 20;
+__host__ __device__ constexpr int vol_geo_stride(int P, bool affine) { return affine ? AFFINE_REC : (5 * P * P + 3) / 4 * 4; }
+
+// Nodal operators of one order, passed by value (constant bank).
+template <int P, typename real>
+struct StageOps {
+  real hatD[P * P], lb0[P], lb1[P], lbw0[P], lbw1[P];
+};
+
+// Elements per group: tiling variant 0 (large groups) and variant 1 (small groups: more CTAs in flight on
+// small meshes); hg_autotune times both on the resident state and keeps the faster.
+__host__ __device__ constexpr int epb_for(int P) { return P == 2 ? 16 : P <= 5 ? 8 : P <= 8 ? 4 : P <= 10 ? 2 : 1; }
+__host__ __device__ constexpr int epb_small_for(int P) { return P <= 3 ? 4 : P <= 5 ? 2 : 1; }
 __host__ __device__ constexpr int epb_stage(int P, int variant) { return variant ? epb_small_for(P) : epb_for(P); }
 __host__ __device__ constexpr int block_of(int P, int EPB) { return ((P * P * EPB + 31) / 32) * 32; }
 __host__ __device__ constexpr int block_for(int P) { return block_of(P, epb_for(P)); }
+// Threads of a stage CTA: the group's face nodes in whole warps (the longest task, one round); small
+// groups also hold a thread per volume node, so that phase A is a single round.
+__host__ __device__ constexpr int stage_threads(int P, int variant) {
+  const int nf = (4 * P * epb_stage(P, variant) + 31) / 32 * 32;
+  return variant ? nf + block_of(P, epb_stage(P, variant)) : nf;
+}
 
 // Four consecutive values of a record that starts at a multiple of 4 values from a cudaMalloc'd base
 // (16-byte aligned in float, 32-byte in double): one 128-bit access in float, two in double.
@@ -104,6 +124,43 @@ __device__ __forceinline__ void cp_async_real(double* dst, const double* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// Four consecutive values from global into shared memory, 16 bytes at a time.
+__device__ __forceinline__ void cp_async_4(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_4(double* dst, const double* src) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + 16u), "l"(src + 2) : "memory");
+}
+
+// Bulk copies (both addresses and the size multiples of 16 bytes) that complete on an mbarrier.
+__device__ __forceinline__ void mbar_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))), "l"(src), "r"(bytes),
+               "r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))) : "memory");
+}
+// Waits for the phase; gives up after a bounded number of polls (each suspends the thread for a while) and
+// reports false, so that a copy which never lands ends the launch instead of hanging it.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
+  const unsigned b = static_cast<unsigned>(__cvta_generic_to_shared(bar));
+  for (int n = 0; n < (1 << 20); ++n) {
+    unsigned done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(b), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
 // max that keeps NaN (a residual that is NaN must stay visible)
 __device__ __forceinline__ double nanmax(double m, double v) { return (v > m || v != v) ? v : m; }
 
@@ -112,7 +169,7 @@ __device__ __forceinline__ double nanmax(double m, double v) { return (v > m || 
 // bit 2 rho <= 0, bit 4 p <= 0 (tested as rho (rho E) - |rho u|^2 / 2 = rho p / (gamma - 1) <= 0, no
 // division).  health = {bits, an offending element (the first to arrive)}; the mapped host flag tells
 // the host without a synchronisation that the word is no longer clean.
-enum { HEALTH_NONFINITE = 1, HEALTH_DENSITY = 2, HEALTH_PRESSURE = 4 };
+enum { HEALTH_NONFINITE = 1, HEALTH_DENSITY = 2, HEALTH_PRESSURE = 4, HEALTH_COPY = 8 };   // COPY: mbar_wait gave up
 __device__ __forceinline__ void check_state(int* health, int* health_host, double r, double ru, double rv,
                                             double rE, int e) {
   const bool finite = fabs(r) + fabs(ru) + fabs(rv) + fabs(rE) < 1.0e300;
@@ -126,234 +183,313 @@ __device__ __forceinline__ void check_state(int* health, int* health_host, doubl
   if (health_host) *reinterpret_cast<volatile int*>(health_host) = 1;
 }
 
-// AFFINE: metrics constant per element (vol_geo [n_el][5]) and normals/dS constant
-// per side (side_geo [n_el*4][3]), as for parallelogram elements with straight edges.
-// LGL: Gauss-Lobatto nodes, whose boundary interpolants are unit vectors (lb = e_0 / e_N): traces are
-// node values and the lift touches only the boundary rows -- the same arithmetic as the dense form
-// with its exact zeros left out.
 __host__ __device__ constexpr int face_node(int P, int side, int l, int kk) {
   return (side == 0 || side == 2) ? (l * P + kk) : (kk * P + l);
 }
-// Order of the P terms of a trace at face node kk: step m takes line node l = (m + kk) mod P.  The face
-// nodes of a side sit in consecutive lanes; without the rotation the lanes of a right or left side (a
-// column of the tile) would read one column at a time, P words apart, into the same banks.  Every Q
-// trace of a state (stage, gradient and trace kernels) sums in this order, so an element's own trace and
-// the copy its neighbour reads stay equal bit for bit.
+// Order of the P terms of a Navier-Stokes trace at face node kk: step m takes line node l = (m + kk) mod P.
+// The face nodes of a side sit in consecutive lanes; without the rotation the lanes of a right or left side
+// (a column of the tile) would read one column at a time, P words apart, into the same banks.
 __host__ __device__ constexpr int trace_l(int P, int m, int kk) { return (m + kk) % P; }
 // The rotation is used in double, where a column side's lanes collide 4 ways; in float they collide 2
 // ways and the rotated (runtime) addressing costs more registers than the conflicts cost time.
 template <typename real>
 __host__ __device__ constexpr int trace_step(int P, int m, int kk) { return sizeof(real) == 8 ? trace_l(P, m, kk) : m; }
 
-template <int P, int EPB, typename real, bool AFFINE, bool LGL>
-__global__ void __launch_bounds__(block_of(P, EPB)) stage_kernel(StageArgs<real> a) {
-  constexpr int NP = P * P;
-  constexpr int FT = 4 * P;
-  constexpr int NW = block_of(P, EPB) / 32;
-  __shared__ real s_mat[NP + 4 * P];
-  __shared__ real s_Fc[4][EPB][NP];
-  __shared__ real s_Gc[4][EPB][NP];
-  __shared__ real s_Q[4][EPB][NP];
-  __shared__ real s_F[4][EPB][FT];
-  __shared__ double s_red[NW][4];
+// Shared memory of a stage CTA.
+template <int P, int V, typename real, bool AFFINE, bool LGL>
+struct StageTiles {
+  static constexpr int EPB = epb_stage(P, V), T = stage_threads(P, V);
+  static constexpr int NP = P * P, FT = 4 * P, PO = P | 1, NN = EPB * NP, NF = EPB * FT, GS = vol_geo_stride(P, AFFINE);
+  static constexpr int VM = sizeof(real) == 8 ? 16 : 32, V0 = EPB * P * PO;
+  static constexpr int VS = V0 + (VM + VM / 4 - V0 % VM) % VM;   // = VM / 4 modulo VM
+  struct In {                       // inputs of one group
+    double Q[NN * 4];
+    real G[NN * 4];
+    real Tn[NF * 4];                // neighbours' traces (or mortar fluxes), in the task's node order
+    real To[LGL ? 4 : NF * 4];      // own traces
+    real vg[EPB * GS];
+    real sg[AFFINE ? 4 : NF * 3];
+  };
+  alignas(16) In in[2];
+  alignas(16) int4 side[3][EPB * 4];
+  real Fc[4 * VS], Gc[4 * VS];      // contravariant fluxes, then their contractions; Fc then holds the new state
+  real F[4 * NF];                   // face fluxes x dS (signed for a RIGHT side)
+  double mx[4][T];                  // per-thread max |QDot|
+  uint64_t bar[2];
+};
 
-  const int flat = threadIdx.x;
-  const int le = flat / NP;               // element in block
-  const int tid = flat - le * NP;         // node in element
-  // hatD held transposed (column l contiguous): conflict-free reads of hatD(i, l) across a warp's nodes
-  for (int k = flat; k < NP + 4 * P; k += blockDim.x) s_mat[k] = real(a.mats[k < NP ? (k % P) * P + k / P : k]);
-  const int e = blockIdx.x * EPB + le;
-  const bool active = le < EPB && e < a.n_el;
+// AFFINE: metrics constant per element and normals / dS constant per side, as for parallelogram elements
+// with straight edges.
+// LGL: Gauss-Lobatto nodes, whose boundary interpolants are unit vectors (lb = e_0 / e_N): traces are
+// node values and the lift touches only the line ends -- the same arithmetic as the dense form with its
+// exact zeros left out.
+template <int P, int V, typename real, bool AFFINE, bool LGL>
+__global__ void __launch_bounds__(stage_threads(P, V))
+    stage_kernel(const __grid_constant__ StageArgs<real> a, const __grid_constant__ StageOps<P, real> op) {
+  using Tl = StageTiles<P, V, real, AFFINE, LGL>;
+  constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, PO = Tl::PO, NF = Tl::NF, VS = Tl::VS, GS = Tl::GS;
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  Tl& s = *reinterpret_cast<Tl*>(stage_smem);
+  const int tid = threadIdx.x;
+  const int n_groups = (a.n_el + EPB - 1) / EPB;
   Phys<real> ph;
   ph.load(a.pc);
-  const int i = tid % P, j = tid / P;
 
-  const size_t off = (size_t(e) * NP + tid) * 4;
-  real geo[5];
-  if (active) {
-    const double2* qp = reinterpret_cast<const double2*>(a.Q + off);
-    const double2 q01 = qp[0], q23 = qp[1];
-    const real q[4] = {real(q01.x), real(q01.y), real(q23.x), real(q23.y)};
-    const real* gp = AFFINE ? a.vol_geo + size_t(e) * 5 : a.vol_geo + (size_t(e) * NP + tid) * 5;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) geo[k] = real(gp[k]);
-    real f[4], g[4];
-    inviscid_flux(ph, q, f, g);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      s_Fc[k][le][tid] = f[k] * geo[0] + g[k] * geo[2];   // F Ja(1,IX) + G Ja(2,IX)
-      s_Gc[k][le][tid] = f[k] * geo[1] + g[k] * geo[3];   // F Ja(1,IY) + G Ja(2,IY)
-      s_Q[k][le][tid] = q[k];
-    }
-  }
-  __syncthreads();
-  const real* hatDT = s_mat;   // transposed: hatDT[l * P + i] = hatD(i, l)
-  const real* lb0 = s_mat + NP;
-  const real* lb1 = lb0 + P;
-  const real* lbw0 = lb1 + P;
-  const real* lbw1 = lbw0 + P;
-
-  // face-node tasks: Riemann fluxes of the 4 sides (element-local order)
-  if (active) {
-    for (int t = tid; t < FT; t += NP) {
-      const int s = t / P, kk = t % P;
-      const int4 sd = a.side[size_t(e) * 4 + s];
+  const auto count = [&](int g) { return min(EPB, a.n_el - g * EPB); };
+  // inputs of group g into half b, and the side table of the group after it (thread 0)
+  const auto issue_bulk = [&](int g, int b, bool own_side, int slot) {
+    const int e0 = g * EPB, n = count(g), gn = g + gridDim.x;
+    const bool rk = a.update && !a.first;
+    typename Tl::In& in = s.in[b];
+    const unsigned bq = n * NP * 32u, bg = rk ? n * NP * 4u * sizeof(real) : 0u, bt = LGL ? 0u : n * FT * 4u * sizeof(real);
+    const unsigned bv = n * GS * unsigned(sizeof(real)), bs = AFFINE ? 0u : n * FT * 3u * sizeof(real);
+    const unsigned b0 = own_side ? n * 64u : 0u, bn = gn < n_groups ? count(gn) * 64u : 0u;
+    uint64_t* bar = &s.bar[b];
+    mbar_expect(bar, bq + bg + bt + bv + bs + b0 + bn);
+    bulk_copy(in.Q, a.Q + size_t(e0) * NP * 4, bq, bar);
+    if (b0) bulk_copy(s.side[slot], a.side + size_t(e0) * 4, b0, bar);
+    if (bt) bulk_copy(in.To, a.T_in + size_t(e0) * FT * 4, bt, bar);
+    bulk_copy(in.vg, a.vol_geo + size_t(e0) * GS, bv, bar);
+    if (bs) bulk_copy(in.sg, a.side_geo + size_t(e0) * FT * 3, bs, bar);
+    if (bg) bulk_copy(in.G, a.G + size_t(e0) * NP * 4, bg, bar);
+    if (bn) bulk_copy(s.side[slot == 2 ? 0 : slot + 1], a.side + size_t(gn) * EPB * 4, bn, bar);
+  };
+  // the neighbours' traces of group g into half b: a face task's copy is issued and read by one thread
+  const auto issue_rows = [&](int g, int b, const int4* side) {
+    const int n = count(g) * FT;
+    for (int x = tid; x < n; x += T) {
+      const int t = x % FT, kk = t % P;
+      const int4 sd = side[(x / FT) * 4 + t / P];
       const int kind = sd.y & 15;
-      if (kind == SIDE_FLUX) {
-        real fp[4];
-        ld4(a.NF + (size_t(sd.x) * P + kk) * 4, fp);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s_F[k][le][t] = fp[k];
-        continue;
-      }
-      const real* lbv = (s == 0 || s == 3) ? lb0 : lb1;
-      real qo[4] = {real(0), real(0), real(0), real(0)};
-      if (LGL) {
-        const int node = face_node(P, s, (s == 0 || s == 3) ? 0 : P - 1, kk);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) qo[k] = s_Q[k][le][node];
-      } else {
-#pragma unroll
-        for (int m = 0; m < P; ++m) {
-          const int l = trace_step<real>(P, m, kk);
-          const int node = face_node(P, s, l, kk);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) qo[k] += s_Q[k][le][node] * lbv[l];
-        }
-      }
-      const real* g3 = AFFINE ? a.side_geo + (size_t(e) * 4 + s) * 3 : a.side_geo + ((size_t(e) * 4 + s) * P + kk) * 3;
-      const real nx = g3[0], ny = g3[1], dS = g3[2];
-      real F[4];
-      if (kind == SIDE_WALL) {
-        euler_wall_flux(ph, qo, nx, ny, dS, F);
-      } else {
-        real qn[4];
-        int solver = a.riemann;
-        if (kind == SIDE_STATE) {
-          const Zone& z = a.zones[sd.z];
-          real us[4];
-          bc_states(ph, z, qo, nx, ny, qn, us, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
-          if (z.riemann >= 0) solver = z.riemann;
-        } else {
-          const int kn = (sd.y & SIDE_REVERSED) ? (P - 1 - kk) : kk;
-          ld4(a.T_in + (size_t(sd.x) * P + kn) * 4, qn);
-          if (sd.z >= 0) { const int zr = a.zones[sd.z].riemann; if (zr >= 0) solver = zr; }
-        }
-        if (kind == SIDE_RIGHT) {
-          face_riemann(solver, ph, qn, qo, nx, ny, a.FX, (size_t(e) * 4 + s) * P + kk, F);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) F[k] = -(F[k] * dS);
-        } else {
-          face_riemann(solver, ph, qo, qn, nx, ny, a.FX, (size_t(e) * 4 + s) * P + kk, F);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) F[k] = F[k] * dS;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) s_F[k][le][t] = F[k];
+      if (kind == SIDE_LEFT || kind == SIDE_RIGHT)
+        cp_async_4(&s.in[b].Tn[x * 4], a.T_in + (size_t(sd.x) * P + ((sd.y & SIDE_REVERSED) ? P - 1 - kk : kk)) * 4);
+      else if (kind == SIDE_FLUX)
+        cp_async_4(&s.in[b].Tn[x * 4], a.NF + (size_t(sd.x) * P + kk) * 4);
     }
-  }
-  __syncthreads();
+    cp_async_commit();
+  };
 
-  real qd[4] = {real(0), real(0), real(0), real(0)};
-  if (active) {
-#pragma unroll
-    for (int l = 0; l < P; ++l) {
-      const real hi = hatDT[l * P + i], hj = hatDT[l * P + j];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) qd[k] = qd[k] + hi * s_Fc[k][le][j * P + l] + hj * s_Gc[k][le][l * P + i];
-    }
-    // lift: bottom F(i) lbw0(j), right F(j) lbw1(i), top F(i) lbw1(j), left F(j) lbw0(i)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (LGL) {
-        if (j == 0) qd[k] = qd[k] - s_F[k][le][0 * P + i] * lbw0[0];
-        if (i == P - 1) qd[k] = qd[k] - s_F[k][le][1 * P + j] * lbw1[P - 1];
-        if (j == P - 1) qd[k] = qd[k] - s_F[k][le][2 * P + i] * lbw1[P - 1];
-        if (i == 0) qd[k] = qd[k] - s_F[k][le][3 * P + j] * lbw0[0];
-      } else {
-        qd[k] = qd[k] - s_F[k][le][0 * P + i] * lbw0[j];
-        qd[k] = qd[k] - s_F[k][le][1 * P + j] * lbw1[i];
-        qd[k] = qd[k] - s_F[k][le][2 * P + i] * lbw1[j];
-        qd[k] = qd[k] - s_F[k][le][3 * P + j] * lbw0[i];
-      }
-      qd[k] = qd[k] * geo[4];
-    }
-    if (a.QDot) {
-      double2* dp = reinterpret_cast<double2*>(a.QDot + off);
-      dp[0] = make_double2(double(qd[0]), double(qd[1]));
-      dp[1] = make_double2(double(qd[2]), double(qd[3]));
-    }
-    if (a.update) {
-      real gn[4];
-      if (a.first) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) gn[k] = real(a.b) * qd[k];
-      } else {
-        real go[4];
-        ld4(a.G + off, go);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) gn[k] = real(a.a) * go[k] + real(a.b) * qd[k];
-      }
-      st4(a.G + off, gn);
-      double2* qp = reinterpret_cast<double2*>(a.Q + off);
-      double2 q01 = qp[0], q23 = qp[1];
-      q01.x = q01.x + a.c * double(gn[0]);
-      q01.y = q01.y + a.c * double(gn[1]);
-      q23.x = q23.x + a.c * double(gn[2]);
-      q23.y = q23.y + a.c * double(gn[3]);
-      qp[0] = q01; qp[1] = q23;
-      check_state(a.health, a.health_host, q01.x, q01.y, q23.x, q23.y, e);
-      s_Q[0][le][tid] = real(q01.x); s_Q[1][le][tid] = real(q01.y);
-      s_Q[2][le][tid] = real(q23.x); s_Q[3][le][tid] = real(q23.y);
-    }
+  if (tid == 0) {
+    mbar_init(&s.bar[0]);
+    mbar_init(&s.bar[1]);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    issue_bulk(blockIdx.x, 0, true, 0);
   }
-  if (a.resid) {   // uniform over the grid: every thread of the CTA takes part
-    double m[4];
+  issue_rows(blockIdx.x, 0, a.side + size_t(blockIdx.x) * EPB * 4);
+  if (a.resid)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) m[k] = active ? fabs(double(qd[k])) : 0.0;
+    for (int k = 0; k < 4; ++k) s.mx[k][tid] = 0.0;
+  __syncthreads();   // the barriers are initialised
+
+  int b = 0, slot = 0;
+  unsigned phase = 0u;
+  for (int g = blockIdx.x; g < n_groups; g += gridDim.x) {
+    const int e0 = g * EPB, n_act = count(g);
+    if (!mbar_wait(&s.bar[b], (phase >> b) & 1u) && tid == 0) {
+      if (a.health) atomicOr(a.health, HEALTH_COPY);
+      if (a.health_host) *reinterpret_cast<volatile int*>(a.health_host) = 1;
+    }
+    phase ^= 1u << b;
+    cp_async_wait_all();
+    __syncthreads();   // every thread is done with the previous group: its half and the work tiles are free
+    const int next_slot = slot == 2 ? 0 : slot + 1;
+    if (g + int(gridDim.x) < n_groups) {
+      if (tid == 0) issue_bulk(g + gridDim.x, b ^ 1, false, next_slot);
+      issue_rows(g + gridDim.x, b ^ 1, s.side[next_slot]);
+    }
+    const typename Tl::In& in = s.in[b];
+    const int4* side = s.side[slot];
+
+    // A: face fluxes and contravariant volume fluxes
+    constexpr int NFR = (NF + 31) / 32 * 32;
+    for (int x = tid; x < NFR + Tl::NN; x += T) {
+      if (x < NFR) {
+        const int le = x / FT, t = x % FT, sd_ = t / P, kk = t % P;
+        if (x >= NF || le >= n_act) continue;
+        const int4 sd = side[le * 4 + sd_];
+        const int kind = sd.y & 15;
+        real qn[4], F[4];
+        if (kind == SIDE_LEFT || kind == SIDE_RIGHT || kind == SIDE_FLUX) ld4(&in.Tn[x * 4], qn);
+        if (kind == SIDE_FLUX) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
+          for (int k = 0; k < 4; ++k) s.F[k * NF + x] = qn[k];
+          continue;
+        }
+        real qo[4];
+        if (LGL) {
+          double qd[4];
+          ld4(&in.Q[(le * NP + face_node(P, sd_, (sd_ == 0 || sd_ == 3) ? 0 : P - 1, kk)) * 4], qd);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) m[k] = nanmax(m[k], __shfl_xor_sync(0xffffffffu, m[k], off));
-    if ((flat & 31) == 0)
+          for (int k = 0; k < 4; ++k) qo[k] = real(qd[k]);
+        } else {
+          ld4(&in.To[x * 4], qo);
+        }
+        const real* g3 = AFFINE ? &in.vg[le * GS + 8 + sd_ * 3] : &in.sg[x * 3];
+        const real nx = g3[0], ny = g3[1], dS = g3[2];
+        if (kind == SIDE_WALL) {
+          euler_wall_flux(ph, qo, nx, ny, dS, F);
+        } else {
+          int solver = a.riemann;
+          if (kind == SIDE_STATE) {
+            const Zone& z = a.zones[sd.z];
+            real us[4];
+            bc_states(ph, z, qo, nx, ny, qn, us, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
+            if (z.riemann >= 0) solver = z.riemann;
+          } else if (sd.z >= 0) {
+            const int zr = a.zones[sd.z].riemann;
+            if (zr >= 0) solver = zr;
+          }
+          const bool right = kind == SIDE_RIGHT;
+          real qL[4], qR[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) s_red[flat >> 5][k] = m[k];
-  }
-  __syncthreads();
-  if (a.resid && flat < 4) {
-    double mx = 0.0;
+          for (int k = 0; k < 4; ++k) { qL[k] = right ? qn[k] : qo[k]; qR[k] = right ? qo[k] : qn[k]; }
+          face_riemann(solver, ph, qL, qR, nx, ny, a.FX, size_t(e0) * FT + x, F);
+          const real sg = right ? -dS : dS;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) mx = nanmax(mx, s_red[w][flat]);
-    a.resid[size_t(blockIdx.x) * 4 + flat] = mx;
-  }
-  // traces of the updated state for the next launch
-  if (active && a.update) {
-    for (int t = tid; t < FT; t += NP) {
-      const int s = t / P, kk = t % P;
-      const real* lbv = (s == 0 || s == 3) ? lb0 : lb1;
-      real tr[4] = {real(0), real(0), real(0), real(0)};
-      if (LGL) {
-        const int node = face_node(P, s, (s == 0 || s == 3) ? 0 : P - 1, kk);
+          for (int k = 0; k < 4; ++k) F[k] *= sg;
+        }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) tr[k] = s_Q[k][le][node];
+        for (int k = 0; k < 4; ++k) s.F[k * NF + x] = F[k];
       } else {
+        const int m = x - NFR, le = m / NP, node = m % NP;
+        if (le >= n_act) continue;
+        double qd[4];
+        ld4(&in.Q[m * 4], qd);
+        const real q[4] = {real(qd[0]), real(qd[1]), real(qd[2]), real(qd[3])};
+        const real* gp = AFFINE ? &in.vg[le * GS] : &in.vg[le * GS + node * 5];
+        const real Ja00 = gp[0], Ja01 = gp[1], Ja10 = gp[2], Ja11 = gp[3];
+        real f[4], gg[4];
+        inviscid_flux(ph, q, f, gg);
+        const int o = (le * P + node / P) * PO + node % P;
 #pragma unroll
-        for (int m = 0; m < P; ++m) {
-          const int l = trace_step<real>(P, m, kk);
-          const int node = face_node(P, s, l, kk);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) tr[k] += s_Q[k][le][node] * lbv[l];
+        for (int k = 0; k < 4; ++k) {
+          s.Fc[k * VS + o] = f[k] * Ja00 + gg[k] * Ja10;   // F Ja(1,IX) + G Ja(2,IX)
+          s.Gc[k * VS + o] = f[k] * Ja01 + gg[k] * Ja11;   // F Ja(1,IY) + G Ja(2,IY)
         }
       }
-      st4(a.T_out + ((size_t(e) * 4 + s) * P + kk) * 4, tr);
+    }
+    __syncthreads();
+
+    // B: contraction and lift, one line of one variable per thread: rows of Fc between the left and right
+    // sides, columns of Gc between the bottom and top ones
+    const auto line = [&](real* U, const int st, const real F0, const real F1) {
+      real in_[P], out[P];
+#pragma unroll
+      for (int l = 0; l < P; ++l) in_[l] = U[l * st];
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        real r = op.hatD[i * P] * in_[0];
+#pragma unroll
+        for (int l = 1; l < P; ++l) r += op.hatD[i * P + l] * in_[l];
+        if (!LGL || i == 0) r -= F0 * op.lbw0[i];
+        if (!LGL || i == P - 1) r -= F1 * op.lbw1[i];
+        out[i] = r;
+      }
+#pragma unroll
+      for (int l = 0; l < P; ++l) U[l * st] = out[l];
+    };
+    for (int x = tid; x < NF; x += T) {   // x = (variable, element, line)
+      const int v = x / (P * EPB), le = (x / P) % EPB, m = x % P;
+      if (le >= n_act) continue;
+      const real* Fv = &s.F[v * NF + le * FT];
+      line(&s.Fc[v * VS + (le * P + m) * PO], 1, Fv[3 * P + m], Fv[P + m]);
+    }
+    for (int x = tid; x < NF; x += T) {
+      const int v = x / (P * EPB), le = (x / P) % EPB, m = x % P;
+      if (le >= n_act) continue;
+      const real* Fv = &s.F[v * NF + le * FT];
+      line(&s.Gc[v * VS + le * P * PO + m], PO, Fv[m], Fv[2 * P + m]);
+    }
+    __syncthreads();
+
+    // C: time derivative and update
+    for (int m = tid; m < n_act * NP; m += T) {
+      const int le = m / NP, node = m % NP, i = node % P, j = node / P;
+      const size_t off = (size_t(e0) * NP + m) * 4;
+      const int o = (le * P + j) * PO + i;
+      const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
+      real qd[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) qd[k] = (s.Fc[k * VS + o] + s.Gc[k * VS + o]) * iJ;
+      if (a.QDot) {
+        const double dq[4] = {double(qd[0]), double(qd[1]), double(qd[2]), double(qd[3])};
+        st4(a.QDot + off, dq);
+      }
+      if (a.resid)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s.mx[k][tid] = nanmax(s.mx[k][tid], fabs(double(qd[k])));
+      if (a.update) {
+        real gn[4];
+        if (a.first) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gn[k] = real(a.b) * qd[k];
+        } else {
+          ld4(&in.G[m * 4], gn);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gn[k] = real(a.a) * gn[k] + real(a.b) * qd[k];
+        }
+        st4(a.G + off, gn);
+        double q[4];
+        ld4(&in.Q[m * 4], q);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = q[k] + a.c * double(gn[k]);
+        st4(a.Q + off, q);
+        check_state(a.health, a.health_host, q[0], q[1], q[2], q[3], e0 + le);
+        const real r[4] = {real(q[0]), real(q[1]), real(q[2]), real(q[3])};
+        if (LGL) {
+          real* tp = a.T_out + size_t(e0 + le) * FT * 4;
+          if (j == 0) st4(tp + i * 4, r);
+          if (i == P - 1) st4(tp + (P + j) * 4, r);
+          if (j == P - 1) st4(tp + (2 * P + i) * 4, r);
+          if (i == 0) st4(tp + (3 * P + j) * 4, r);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) s.Fc[k * VS + o] = r[k];
+        }
+      }
+    }
+
+    // D: traces of the new state at both ends of every line; the variable runs fastest over the lanes, so
+    // that four of them write one 4-value record
+    if (!LGL && a.update) {
+      __syncthreads();
+      const auto ends = [&](const real* U, const int st, real* t0, real* t1) {
+        real r0 = real(0), r1 = real(0);   // summed as trace_kernel does, bit for bit
+#pragma unroll
+        for (int l = 0; l < P; ++l) {
+          const real u = U[l * st];
+          r0 += op.lb0[l] * u;
+          r1 += op.lb1[l] * u;
+        }
+        *t0 = r0;
+        *t1 = r1;
+      };
+      for (int x = tid; x < n_act * FT; x += T) {   // x = (element, line, variable)
+        const int v = x & 3, le = x / FT, m = (x >> 2) % P;
+        real* tp = a.T_out + size_t(e0 + le) * FT * 4 + v;
+        ends(&s.Fc[v * VS + (le * P + m) * PO], 1, tp + (3 * P + m) * 4, tp + (P + m) * 4);
+        ends(&s.Fc[v * VS + le * P * PO + m], PO, tp + m * 4, tp + (2 * P + m) * 4);
+      }
+    }
+    b ^= 1;
+    slot = next_slot;
+  }
+  if (a.resid) {
+    __syncthreads();
+    if (tid < 4) {
+      double m = 0.0;
+      for (int t = 0; t < T; ++t) m = nanmax(m, s.mx[tid][t]);
+      a.resid[size_t(blockIdx.x) * 4 + tid] = m;
     }
   }
 }
 
 // Traces of the resident state (after hg_set_state).
+// rotated: the summation order of the Navier-Stokes stage kernels (trace_step), else that of the Euler
+// stage kernel, so that a state loaded from the host has the traces bit for bit that a stage left.
 template <int P, int EPB, typename real>
-__global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const double* Q, const double* mats, real* T) {
+__global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const double* Q, const double* mats, real* T,
+                                                             bool rotated) {
   constexpr int NP = P * P;
   constexpr int FT = 4 * P;
   __shared__ real s_lb[2 * P];
@@ -373,7 +509,7 @@ __global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const dou
     const real* lbv = (s == 0 || s == 3) ? s_lb : s_lb + P;
     real tr[4] = {real(0), real(0), real(0), real(0)};
     for (int m = 0; m < P; ++m) {
-      const int l = trace_step<real>(P, m, kk);
+      const int l = rotated ? trace_step<real>(P, m, kk) : m;
       const int node = face_node(P, s, l, kk);
 #pragma unroll
       for (int k = 0; k < 4; ++k) tr[k] += s_Q[k][le][node] * lbv[l];
