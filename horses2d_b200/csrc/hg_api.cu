@@ -53,7 +53,7 @@ void ctx_free(hg_ctx* c) {
   drop_graph(c);
   for (cudaEvent_t e : c->prof_pool) cudaEventDestroy(e);
   void* ptrs[] = {c->d_side, c->d_side_geo, c->d_vol_geo, c->d_mats, c->d_zones, c->d_Q, c->d_G, c->d_T[0], c->d_T[1],
-                  c->d_QDot, c->d_resid, c->d_resid_out, c->d_elmax, c->d_side_invh, c->d_jac, c->d_GT[0],
+                  c->d_QDot, c->d_resid, c->d_resid_out, c->d_elmax, c->d_side_invh, c->d_face_metric, c->d_GT[0],
                   c->d_GT[1], c->d_av_el, c->d_side_area, c->d_mu_av[0], c->d_mu_av[1], c->d_mlp, c->d_feat_lo,
                   c->d_feat_hi, c->d_dQ,
                   c->d_FX, c->d_bq, c->d_si_out, c->d_NF, c->d_NFG, c->d_NJ, c->d_exact_sides};
@@ -119,21 +119,20 @@ static void health_check(hg_ctx* c) {
                 "); set a new state to continue");
 }
 
-// Tiling of the Euler stage kernel: variant 0's groups of elements are cut to variant 1's where they would
+// Tiling of the stage kernels: variant 0's groups of elements are cut to variant 1's where they would
 // leave half of the SMs or more without one (fewer than two groups per SM): there a stage is one pass of
 // latency, and the smaller groups spread it over the chip.
+// (Navier-Stokes orders 9 and 10 run one element per group in both variants, one instantiation.)
 static int stage_variant(const hg_ctx* c, int variant) {
-  return variant || c->n_el < 2 * c->n_sm * epb_stage(c->P, 0) ? 1 : 0;
+  if (c->ns && c->P >= 10) return 0;
+  return variant || c->n_el < 2 * c->n_sm * (c->ns ? epb_ns_of(c->P, 0) : epb_stage(c->P, 0)) ? 1 : 0;
 }
 static int epb_of(const hg_ctx* c, int variant) {
-  return c->ns ? epb_ns_of(c->P, variant) : epb_stage(c->P, stage_variant(c, variant));
+  const int v = stage_variant(c, variant);
+  return c->ns ? epb_ns_of(c->P, v) : epb_stage(c->P, v);
 }
-// per-CTA residual partials: room for the tiling variant with the most CTAs
-static int max_grid(const hg_ctx* c) {
-  if (!c->ns) return std::min(c->n_el, 32 * c->n_sm);
-  const int epb = std::min(epb_of(c, 0), epb_of(c, 1));
-  return (c->n_el + epb - 1) / epb;
-}
+// per-CTA residual partials
+static int max_grid(const hg_ctx* c) { return std::min(c->n_el, 32 * c->n_sm); }
 
 #define HG_DISPATCH_P(P_, FN, ...)                      \
   switch (P_) {                                         \
@@ -171,9 +170,10 @@ static void run_trace(hg_ctx* c) { HG_DISPATCH_P_EULER(c->P, launch_trace_P, c);
 
 template <int P, typename real>
 static void ns_dispatch(hg_ctx* c, const NSArgs<real>& a) {
-  // orders 9-10 run one element per CTA in both tilings: one instantiation serves
-  if (c->tiling && P < 10) launch_ns_PV<P, real, 1>(c, a);
-  else launch_ns_PV<P, real, 0>(c, a);
+  if constexpr (P < 10) {
+    if (stage_variant(c, c->tiling)) { launch_ns_PV<P, real, 1>(c, a); return; }
+  }
+  launch_ns_PV<P, real, 0>(c, a);
 }
 
 // Navier-Stokes kernels: orders 1-8, 9 and 10
@@ -205,8 +205,7 @@ static void run_ns_stage(hg_ctx* c, double ca, double cb, double cc, bool first,
   a.side_geo = static_cast<const real*>(c->d_side_geo);
   a.side_invh = c->d_side_invh;
   a.vol_geo = static_cast<const real*>(c->d_vol_geo);
-  a.jac = static_cast<const real*>(c->d_jac);
-  a.mats = c->d_mats;
+  a.face_metric = static_cast<const real*>(c->d_face_metric);
   a.zones = c->d_zones;
   a.bq = c->d_bq;
   a.FX = static_cast<const real*>(c->d_FX);
@@ -221,10 +220,10 @@ static void run_ns_stage(hg_ctx* c, double ca, double cb, double cc, bool first,
   a.GT_out = static_cast<real*>(c->d_GT[c->cur ^ 1]);
   a.dQ = static_cast<real*>(c->d_dQ);
   a.viscous = (c->pc.mu != 0.0 || c->av == HG_AV_PHYSICAL) ? 1 : 0;
-  // BR1 always needs the lifted gradient; IP only for gradient traces (viscous fluxes) or the indicator
-  // (the jumps indicator every stage, the modal and learned ones on the first stage of a step)
-  a.run_gradient = (!c->ip || a.viscous ||
-                    (c->av != HG_AV_NONE && (c->sensor_kind == HG_SENSOR_JUMPS || first))) ? 1 : 0;
+  // BR1 always needs the lifted gradient; IP only for gradient traces (viscous fluxes) or the modal and
+  // learned indicators on the first stage of a step; the jumps indicator has its own kernel every stage
+  a.run_jumps = (c->av != HG_AV_NONE && c->sensor_kind == HG_SENSOR_JUMPS) ? 1 : 0;
+  a.run_gradient = (!c->ip || a.viscous || (c->av != HG_AV_NONE && !a.run_jumps && first)) ? 1 : 0;
   a.QDot = qdot;
   a.resid = resid ? c->d_resid : nullptr;
   a.a = ca; a.b = cb; a.c = cc;
@@ -246,7 +245,7 @@ static void run_ns_stage(hg_ctx* c, double ca, double cb, double cc, bool first,
   a.health = c->d_health;
   a.health_host = c->d_health_flag;
   a.run_stage = c->ns_phase != 1;
-  if (c->ns_phase == 2) a.run_gradient = 0;
+  if (c->ns_phase == 2) a.run_gradient = a.run_jumps = 0;
   a.fuse = (ns_fused(c) && !c->prologue) ? 1 : 0;
   a.last = c->last_stage ? 1 : 0;
   if (a.fuse) a.run_gradient = 0;   // the previous stage (or the prologue) left GT and mu_av of this state
@@ -678,8 +677,23 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
     for (auto& g_ : c->d_GT) g_ = dalloc<char>(size_t(E) * 4 * P * 8 * rs);
     c->d_dQ = dalloc<char>(size_t(c->ndof) * 2 * rs);
     HG_CUDA(cudaMemcpy(c->d_side_invh, sinvh.data(), sinvh.size() * sizeof(double), cudaMemcpyHostToDevice));
-    if (!c->affine) {
-      upload_real(c->d_jac, m->jac, size_t(E) * NP);
+    if (!c->affine && c->grad_faces) {
+      // metrics over the jacobian at the side nodes, both interpolated along the normal line
+      std::vector<double> fm(size_t(E) * 4 * P * 4);
+      for (int e = 0; e < E; ++e)
+        for (int sd = 0; sd < 4; ++sd) {
+          const std::vector<double>& lb = (sd == 0 || sd == 3) ? ops.lb0 : ops.lb1;
+          for (int kk = 0; kk < P; ++kk) {
+            double v[5] = {};
+            for (int l = 0; l < P; ++l) {
+              const size_t n = size_t(e) * NP + face_node(P, sd, l, kk);
+              for (int k = 0; k < 4; ++k) v[k] += lb[l] * m->Ja[n * 4 + k];
+              v[4] += lb[l] * m->jac[n];
+            }
+            for (int k = 0; k < 4; ++k) fm[((size_t(e) * 4 + sd) * P + kk) * 4 + k] = v[k] / v[4];
+          }
+        }
+      upload_real(c->d_face_metric, fm.data(), fm.size());
     }
   }
   if (c->riemann == HG_RIEMANN_EXACT) c->exact = true;
@@ -1568,7 +1582,8 @@ extern "C" int hg_get_tiling(const hg_ctx* c, int32_t out[3]) {
   const int epb = epb_of(c, c->tiling);
   out[0] = c->tiling;
   out[1] = epb;
-  out[2] = c->ns ? block_of(c->P, epb) : stage_threads(c->P, stage_variant(c, c->tiling));
+  const int v = stage_variant(c, c->tiling);
+  out[2] = c->ns ? ns_threads(c->P, v) : stage_threads(c->P, v);
   return 0;
 }
 

@@ -66,32 +66,81 @@ void launch_trace_P(hg_ctx* c) {
   const int grid = (c->n_el + EPB - 1) / EPB;
   timed(c, HG_KERNEL_TRACE, [&] {
     trace_kernel<P, EPB, real><<<grid, block_for(P), 0, c->stream>>>(c->n_el, c->d_Q, c->d_mats,
-                                                                     static_cast<real*>(c->d_T[c->cur]), c->ns);
+                                                                     static_cast<real*>(c->d_T[c->cur]),
+                                                                     c->ns ? (c->ip ? TRACE_PLAIN : TRACE_RELATIVE)
+                                                                           : c->node_type == HG_NODES_LGL ? TRACE_NODAL : TRACE_PLAIN);
   });
   ++c->launches;
 }
 
+template <int P, typename real>
+static NSOps<P, real> ns_ops(const hg_ctx* c) {
+  NSOps<P, real> o;
+  const double* m = c->h_mats.data();   // hatD lb0 lb1 lbw0 lbw1 D dlbw0 dlbw1 w Vinv
+  const auto put = [&](real* d, int n) {
+    for (int k = 0; k < n; ++k) d[k] = real(m[k]);
+    m += n;
+  };
+  const double *lb = m + P * P, *D = m + P * P + 4 * P;
+  for (int l = 0; l < P; ++l) {
+    double d0 = 0.0, d1 = 0.0;
+    for (int i = 0; i < P; ++i) {
+      d0 += lb[i] * D[i * P + l];
+      d1 += lb[P + i] * D[i * P + l];
+    }
+    o.dl0[l] = real(d0);
+    o.dl1[l] = real(d1);
+  }
+  put(o.hatD, P * P);
+  put(o.lb0, P); put(o.lb1, P); put(o.lbw0, P); put(o.lbw1, P);
+  put(o.D, P * P);
+  put(o.dlbw0, P); put(o.dlbw1, P); put(o.w, P);
+  put(o.Vinv, P * P);
+  return o;
+}
+
+// Persistent launch of a Navier-Stokes kernel with tiles Tl; returns its CTAs.
+template <typename Tl, typename K, typename A, typename O>
+static int launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind, bool weights, const A& a, const O& op) {
+  static_assert(sizeof(Tl) + MLP_BYTES <= 227 * 1024, "shared memory of a CTA");
+  const size_t smem = sizeof(Tl) + (weights ? MLP_BYTES : 0);
+  const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
+  const int most = c->n_sm * std::min(32, resident_ctas(c, known, kernel, Tl::T, smem));
+  const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
+  timed(c, kind, [&] { kernel<<<grid, Tl::T, smem, c->stream>>>(a, op); });
+  ++c->launches;
+  return grid;
+}
+
 template <int P, typename real, int V, bool AFFINE, bool IP, bool AV>
 static void launch_ns_PAI(hg_ctx* c, const NSArgs<real>& a) {
-  constexpr int EPB = epb_ns_of(P, V);
-  constexpr int BLK = block_of(P, EPB);
-  const int grid = (a.n_el + EPB - 1) / EPB;
-  static bool attr = false;
-  if (!attr) {
-    max_carveout(ns_gradient_kernel<P, EPB, real, AFFINE, IP, AV>);
-    max_carveout(ns_stage_kernel<P, EPB, real, AFFINE, IP, AV>);
-    attr = true;
-  }
+  const NSOps<P, real> op = ns_ops<P, real>(c);
+  const bool learned = AV && a.sensor.kind == SENSOR_LEARNED;
   if (a.run_gradient) {
-    timed(c, HG_KERNEL_GRADIENT,
-          [&] { ns_gradient_kernel<P, EPB, real, AFFINE, IP, AV><<<grid, BLK, 0, c->stream>>>(a); });
+    using Tl = NSTiles<P, V, real, AFFINE, IP, AV, true, true>;
+    static std::atomic<int> known[2][HG_KNOWN_DEVICES];
+    launch_groups<Tl>(c, known[learned], ns_gradient_kernel<P, V, real, AFFINE, IP, AV>, HG_KERNEL_GRADIENT, learned, a, op);
+  }
+  if (AV && a.run_jumps) {
+    EdgeWeights<P, real> ew;
+    for (int k = 0; k < P; ++k) ew.w[k] = op.w[k];
+    const int grid = (a.n_el + jumps_epb(P) - 1) / jumps_epb(P);
+    timed(c, HG_KERNEL_GRADIENT, [&] { jumps_kernel<P, real, AFFINE><<<grid, 128, 0, c->stream>>>(a, ew); });
     ++c->launches;
   }
   if (a.run_stage) {
+    const bool w = learned && a.fuse && a.update && a.last;
+    int grid;
+    if (!AV || a.viscous) {
+      using Tl = NSTiles<P, V, real, AFFINE, IP, AV, true, false>;
+      static std::atomic<int> known[2][HG_KNOWN_DEVICES];
+      grid = launch_groups<Tl>(c, known[w], ns_stage_kernel<P, V, real, AFFINE, IP, AV, true>, HG_KERNEL_STAGE, w, a, op);
+    } else {
+      using Tl = NSTiles<P, V, real, AFFINE, IP, AV, !AV, false>;
+      static std::atomic<int> known[2][HG_KNOWN_DEVICES];
+      grid = launch_groups<Tl>(c, known[w], ns_stage_kernel<P, V, real, AFFINE, IP, AV, !AV>, HG_KERNEL_STAGE, w, a, op);
+    }
     if (a.resid) c->n_resid = grid;
-    timed(c, HG_KERNEL_STAGE,
-          [&] { ns_stage_kernel<P, EPB, real, AFFINE, IP, AV><<<grid, BLK, 0, c->stream>>>(a); });
-    ++c->launches;
   }
 }
 
@@ -116,44 +165,60 @@ void launch_ns_PV(hg_ctx* c, const NSArgs<real>& a) {
 // Sensor indicators of the resident state, per element: features [n_el][16] (optional) and
 // {modal G, learned G, out-of-distribution flag, G used} [n_el][4] (optional).  The learned G is
 // evaluated whenever weights are set.
-template <int P, int EPB, typename real>
-__global__ void __launch_bounds__(block_ns(P)) sensor_eval_kernel(int n_el, const double* Q, const double* mats,
-                                                                  SensorArgs sa, PhysConst pc, float* feat,
-                                                                  double* out) {
-  constexpr int NP = P * P;
-  __shared__ real sQ[4][EPB][NP];
-  __shared__ real sV[NP];
-  const int flat = threadIdx.x, le = flat / NP, tid = flat - le * NP;
-  const int e = blockIdx.x * EPB + le;
-  const bool active = le < EPB && e < n_el;
-  for (int k = flat; k < NP; k += blockDim.x) sV[k] = real(mats[2 * NP + 7 * P + k]);
-  if (active) {
-    const double* q = Q + (size_t(e) * NP + tid) * 4;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) sQ[k][le][tid] = real(q[k]);
+template <int P, typename real>
+struct SensorTiles {
+  static constexpr int EPB = epb_ns(P), T = ns_threads(P, 0), V0 = EPB * P * (P | 1);
+  static constexpr int VM = sizeof(real) == 8 ? 16 : 32, VS = V0 + (VM + VM / 4 - V0 % VM) % VM;
+  alignas(16) real Q[4 * VS];
+  real U[2 * VS];
+  alignas(16) real scr[T / 32 * sensor_scratch(P)];
+  alignas(16) float w[MLP_PARAMS];
+};
+template <int P, typename real>
+struct SensorOps { real Vinv[P * P]; };
+template <int P, typename real>
+__global__ void __launch_bounds__(ns_threads(P, 0)) sensor_eval_kernel(int n_el, const double* Q, const __grid_constant__ SensorOps<P, real> op,
+                                                                       SensorArgs sa, PhysConst pc, float* feat,
+                                                                       double* out) {
+  using Tl = SensorTiles<P, real>;
+  constexpr int NP = P * P, PO = P | 1;
+  extern __shared__ __align__(16) unsigned char sensor_smem[];
+  Tl& s = *reinterpret_cast<Tl*>(sensor_smem);
+  const int tid = threadIdx.x, e0 = blockIdx.x * Tl::EPB, n_act = min(Tl::EPB, n_el - e0);
+  SensorArgs s2 = sa;
+  if (sa.mlp) {
+    s2.kind = SENSOR_LEARNED;
+    sensor_weights_async(s.w, sa.mlp, tid, Tl::T);
   }
+  for (int m = tid; m < n_act * NP; m += Tl::T)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s.Q[k * Tl::VS + (m / P) * PO + m % P] = real(Q[(size_t(e0) * NP + m) * 4 + k]);
+  cp_async_wait_all();
   __syncthreads();
   Phys<real> ph;
   ph.load(pc);
-  SensorArgs s2 = sa;
-  if (sa.mlp) s2.kind = SENSOR_LEARNED;
-  const int n_active = n_el - int(blockIdx.x) * EPB < EPB ? n_el - int(blockIdx.x) * EPB : EPB;
-  SensorOut so = element_sensor<P, EPB, real>(s2, ph, sQ, n_active, sV, le, tid, active,
-                                             (active && feat) ? feat + size_t(e) * MLP_IN : nullptr);
-  if (active && tid == 0 && out) {
-    const double g = sa.kind == SENSOR_LEARNED ? so.g : (sa.kind == SENSOR_MODAL ? so.g_modal : -1.0);
-    out[size_t(e) * 4 + 0] = so.g_modal;
-    out[size_t(e) * 4 + 1] = sa.mlp ? so.g_learned : -1.0;
-    out[size_t(e) * 4 + 2] = so.ood;
-    out[size_t(e) * 4 + 3] = g;
-  }
+  FlatG flat_g;
+  group_sensor<P, Tl::EPB, Tl::T, real>(s2, ph, op.Vinv, s.Q, s.U, Tl::VS, s.scr, s.w, n_act, tid,
+                                        feat ? feat + size_t(e0) * MLP_IN : nullptr, flat_g,
+                                        [&](int le, double gm, double gl, bool ood, double) {
+                                          if (!out) return;
+                                          double* o = out + size_t(e0 + le) * 4;
+                                          o[0] = gm;
+                                          o[1] = sa.mlp ? gl : -1.0;
+                                          o[2] = ood ? 1.0 : 0.0;
+                                          o[3] = sa.kind == SENSOR_JUMPS ? -1.0 : sa.kind == SENSOR_LEARNED && !ood ? gl : gm;
+                                        });
 }
 
 template <int P, typename real>
 void launch_sensor_eval_P(hg_ctx* c, float* feat, double* out) {
-  constexpr int EPB = epb_ns(P);
-  const int grid = (c->n_el + EPB - 1) / EPB;
-  sensor_eval_kernel<P, EPB, real><<<grid, block_ns(P), 0, c->stream>>>(c->n_el, c->d_Q, c->d_mats, sensor_args(c),
-                                                                         c->pc, feat, out);
+  using Tl = SensorTiles<P, real>;
+  static std::atomic<int> known[HG_KNOWN_DEVICES];
+  resident_ctas(c, known, sensor_eval_kernel<P, real>, Tl::T, sizeof(Tl));   // allows the shared memory
+  SensorOps<P, real> op;
+  const double* vinv = c->h_mats.data() + 2 * P * P + 7 * P;
+  for (int k = 0; k < P * P; ++k) op.Vinv[k] = real(vinv[k]);
+  const int grid = (c->n_el + Tl::EPB - 1) / Tl::EPB;
+  sensor_eval_kernel<P, real><<<grid, Tl::T, sizeof(Tl), c->stream>>>(c->n_el, c->d_Q, op, sensor_args(c), c->pc, feat, out);
   ++c->launches;
 }

@@ -1,29 +1,32 @@
 // hg_ns.cuh -- Navier-Stokes stage kernels (BR1 and interior penalty) for sm_100a.
 //
-// Per Runge-Kutta stage two launches:
-//   ns_gradient_kernel  the element gradient dQ -- BR1 lifting
+// Launches per Runge-Kutta stage:
+//   ns_gradient_kernel  BR1: the lifted gradient
 //        dQ = [ -VolGreen(Q Ja) + sum_faces lift(u* dS n) ] / J,  u* = (QL + QR)/2 or the
 //        boundary's viscous state (BR1_ComputeGradient, Approximation/DGViscous_BR1.f90:48-111;
-//        ComputeSolutionRiemann_*, DGViscousMethods.f90:538-917), or the interior-penalty local
-//        gradient (ComputeInteriorGradient, Mesh/QuadElement_QuadProcedures.incf:42-88) -- and
-//        writes only its traces on the four sides (interpolateGradientsToBoundaries,
-//        DGSpatialDiscretizationMethods.f90:1577-1631);
-//   ns_gradient_kernel also stores the BR1 gradient dQ ([n_el][2][4][NP], coalesced per node); the
-//        interior-penalty gradient is element-local and the stage kernel recomputes it, so with IP the
-//        gradient kernel runs only when something else needs it (gradient traces for viscous fluxes,
-//        the artificial-viscosity indicator);
-//   interior penalty with an element-local indicator (none, modal, learned): no gradient kernel per
-//        stage.  The stage kernel ends with the gradient traces of the state it wrote (GT_out, the
-//        other half of a ping-pong pair, as for the Q traces) and, on the last stage of a time step,
-//        the indicator of that state (mu_next): everything the next stage reads from its neighbours.
-//        The gradient kernel then runs only once after the state is replaced (hg_set_state);
-//   ns_stage_kernel     reads the BR1 dQ back (written once, read once per stage),
-//        F = Fi - Fv at the nodes (QDotVolumeLoop :243-268), face fluxes
-//        F* = (Fi* - Fv*) dS with the neighbours' Q and dQ traces (BR1: (FvL+FvR)/2 . n; IP adds
-//        sigma0 mu N^2 invh (uL - uR), DGViscous_IP.f90:45-130), boundary viscous fluxes by
-//        condition (Dirichlet / adiabatic / Neumann, :1142-1511), the interior-penalty gradient-face
-//        terms lifted by Scalar_StdGradientFace (DGWeakIntegrals.f90:268-495), 1/J, the RK update
-//        and the new Q traces.
+//        ComputeSolutionRiemann_*, DGViscousMethods.f90:538-917), stored ([n_el][2][4][NP]) with its traces on
+//        the four sides (interpolateGradientsToBoundaries, DGSpatialDiscretizationMethods.f90:1577-1631);
+//        interior penalty: the traces of the local gradient (ComputeInteriorGradient,
+//        Mesh/QuadElement_QuadProcedures.incf:42-88) and the element-local indicator -- only as the prologue
+//        after the state is replaced (hg_set_state), or per stage on a mixed-order mesh;
+//   jumps_kernel        the reference's interface-jumps indicator, from the traces alone;
+//   ns_stage_kernel     F = Fi - Fv at the nodes (QDotVolumeLoop :243-268), face fluxes F* = (Fi* - Fv*) dS
+//        with the neighbours' Q and dQ traces (BR1: (FvL+FvR)/2 . n; IP adds sigma0 mu N^2 invh (uL - uR),
+//        DGViscous_IP.f90:45-130), boundary viscous fluxes by condition (Dirichlet / adiabatic / Neumann,
+//        :1142-1511), the interior-penalty gradient-face terms lifted by Scalar_StdGradientFace
+//        (DGWeakIntegrals.f90:268-495), 1/J, the RK update and the new Q traces.  Interior penalty with an
+//        element-local indicator (none, modal, learned): it ends with the gradient traces of the state it
+//        wrote (GT_out, the other half of a ping-pong pair, as for the Q traces) and, on the last stage of
+//        a time step, the indicator of that state (mu_next): everything the next stage reads from its
+//        neighbours, so a stage is this one launch.
+//
+// Both kernels are built like the Euler stage kernel (hg_stage.cuh): persistent CTAs over groups of EPB
+// elements with the next group's inputs in flight, and inside a group phases over items (face nodes, volume
+// nodes, lines) between barriers.  Every product with a nodal operator is a line: one thread holds the P
+// nodes of a (variable, line) in registers and takes the operator from the constant bank.  The kernels before
+// held one node per thread and read the operators and the tiles from shared memory, 1.25 loads per
+// multiply-add: their shared-memory pipe ran at 78-81 % of its peak at N = 7 with a quarter of the FP64 rate
+// used, and a third of the warps' time went into global loads at the phase that needed them.
 #pragma once
 #include "hg_stage.cuh"
 #include "hg_sensor.cuh"
@@ -37,8 +40,7 @@ struct NSArgs {
   const real* side_geo;     // normals / dS (per node, or per side when AFFINE)
   const double* side_invh;  // [n_el*4] invh of the side's edge
   const real* vol_geo;      // element records of vol_geo_stride reals (hg_stage.cuh)
-  const real* jac;          // [n_el][NP] J per node (curved meshes)
-  const double* mats;       // hatD[NP] lb0 lb1 lbw0 lbw1 [P each] D[NP] dlbw0 dlbw1 [P each]
+  const real* face_metric;  // [n_el*4][P][4] Ja00/J Ja01/J Ja10/J Ja11/J at the side nodes (curved, gradient faces)
   const Zone* zones;
   const double* bq;         // per-node Dirichlet states [rows][P][4] (sides whose side.w >= 0)
   const real* FX;           // exact-solver face fluxes [n_el*4][P][4] of this stage (RIEMANN_EXACT faces)
@@ -54,6 +56,7 @@ struct NSArgs {
   real* dQ;                 // element gradients              [n_el][2][4][NP]
   int viscous;              // viscous fluxes present: mu != 0 or the Physical artificial viscosity
   int run_gradient;         // host side: whether this stage needs the gradient kernel
+  int run_jumps;            // host side: whether it needs the jumps kernel
   int run_stage;            // host side: whether to launch the stage kernel (a composite runs the
                             // mortar fluxes between the parts' gradient and stage kernels)
   double* QDot;
@@ -67,7 +70,7 @@ struct NSArgs {
   int av;                   // 0 none, 1 Laplacian, 2 Physical
   const double* av_el;      // [n_el][2] Ceps sqrt(Volume)/(N+1), sum of the 4 edge areas
   const double* side_area;  // [n_el*4] Area of each side's edge
-  double* mu_av;            // [n_el] element viscosity of the current state (written by the gradient kernel)
+  double* mu_av;            // [n_el] element viscosity of the current state (written by the gradient or jumps kernel)
   SensorArgs sensor;        // which indicator sets it (jumps, modal, learned)
   int fuse;                 // interior penalty, element-local indicator: the stage kernel writes GT_out and,
   int last;                 //   on the last stage of a step (last), the indicator of its new state into
@@ -76,272 +79,406 @@ struct NSArgs {
   int* health_host;         // mapped host flag set beside it
 };
 
-__host__ __device__ constexpr int epb_ns(int P) {
-  return P == 2 ? 16 : P == 3 ? 7 : P == 4 ? 8 : P == 5 ? 5 : P == 6 ? 4 : P == 7 ? 3 : P <= 9 ? 2 : 1;
-}
-__host__ __device__ constexpr int epb_ns_small(int P) {
-  return P == 2 ? 4 : P <= 6 ? 2 : 1;
-}
+// Elements per group and threads per CTA: variant 0, and variant 1 for small meshes.
+__host__ __device__ constexpr int epb_ns(int P) { return P == 2 ? 16 : P <= 4 ? 8 : P <= 6 ? 4 : P <= 8 ? 2 : 1; }
+__host__ __device__ constexpr int epb_ns_small(int P) { return P <= 3 ? 4 : P <= 6 ? 2 : 1; }
 __host__ __device__ constexpr int epb_ns_of(int P, int variant) { return variant ? epb_ns_small(P) : epb_ns(P); }
-__host__ __device__ constexpr int block_ns(int P) { return ((P * P * epb_ns(P) + 31) / 32) * 32; }
+__host__ __device__ constexpr int ns_threads(int P, int variant) {
+  return (cmax(P * P, 4 * P) * epb_ns_of(P, variant) + 31) / 32 * 32;
+}
 
-// Shared tiles of one CTA.
-// ST: the stage kernel's tiles; the gradient kernel has no contravariant fluxes (Fc, Gc) and leaves
-// that shared memory to the shock sensor.
-template <int P, int EPB, typename real, bool AFFINE, bool ST = true>
-struct NSTiles {
-  static constexpr int NP = P * P, FT = 4 * P;
-  real mat[3 * NP + 7 * P];   // hatD lb0 lb1 lbw0 lbw1 D dlbw0 dlbw1 w Vinv
-  real Q[4][EPB][NP];
-  real Ja[AFFINE ? 1 : 5][AFFINE ? 1 : EPB][AFFINE ? 1 : NP];   // Ja00 Ja01 Ja10 Ja11 J
-  real dQ[2][4][EPB][NP];
-  real Fc[ST ? 4 : 1][ST ? EPB : 1][ST ? NP : 1];
-  real Gc[ST ? 4 : 1][ST ? EPB : 1][ST ? NP : 1];
-  real face[12][EPB][FT];   // BR1 u* dS n (8) / F* (4) + gradient-face contravariant fluxes (8)
-  real gfd[ST ? 4 : 1][ST ? EPB : 1][ST ? FT : 1];   // gradient-face terms contracted along their side
-  real dl[ST && AFFINE ? 2 : 1][ST && AFFINE ? P : 1];   // (lb0^T D)(l), (lb1^T D)(l): normal derivatives at the sides
-  double red[32][4];
+// Nodal operators, passed by value (constant bank); dl = lb^T D, the normal derivatives at the sides.
+template <int P, typename real>
+struct NSOps {
+  real hatD[P * P], D[P * P], lb0[P], lb1[P], lbw0[P], lbw1[P], dlbw0[P], dlbw1[P], dl0[P], dl1[P], w[P], Vinv[P * P];
 };
 
-template <int P, int EPB, typename real, bool AFFINE, bool ST>
-__device__ __forceinline__ real trace_of(const NSTiles<P, EPB, real, AFFINE, ST>& s, const real (*src)[EPB][P * P], int k,
-                                         int le, int side, int kk, const real* lbv) {
-  real t = real(0);
+// out = M in, row by row
+template <int P, typename real>
+__device__ __forceinline__ void apply(const real* M, const real (&in)[P], real (&out)[P]) {
 #pragma unroll
-  for (int m = 0; m < P; ++m) {
-    const int l = trace_step<real>(P, m, kk);
-    t += src[k][le][face_node(P, side, l, kk)] * lbv[l];
-  }
-  return t;
-}
-
-// The four variables' traces at face node kk of side `side` (the interpolant weights loaded once).
-template <int P, int EPB, typename real>
-__device__ __forceinline__ void trace4(const real (*src)[EPB][P * P], int le, int side, int kk, const real* lbv,
-                                       real* out) {
+  for (int i = 0; i < P; ++i) {
+    real r = real(0);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) out[k] = real(0);
-#pragma unroll
-  for (int m = 0; m < P; ++m) {
-    const int l = trace_step<real>(P, m, kk);
-    const int node = face_node(P, side, l, kk);
-    const real w = lbv[l];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) out[k] += src[k][le][node] * w;
+    for (int l = 0; l < P; ++l) r += M[i * P + l] * in[l];
+    out[i] = r;
   }
 }
+template <int P, typename real>
+__device__ __forceinline__ real dot(const real* c, const real (&in)[P]) {
+  real r = real(0);
+#pragma unroll
+  for (int l = 0; l < P; ++l) r += c[l] * in[l];
+  return r;
+}
+// The state's trace at an end of a line (boundary interpolant c, which sums to 1) for BR1.  In float relative to
+// the line's first node, so that the products round a difference; trace_kernel sums the same way.
+template <int P, typename real>
+__device__ __forceinline__ real trace_dot(const real* c, const real (&in)[P]) {
+  if (sizeof(real) == 8) return dot<P>(c, in);
+  real r = real(0);
+#pragma unroll
+  for (int l = 1; l < P; ++l) r += c[l] * (in[l] - in[0]);
+  return in[0] + r;
+}
+template <int P, typename real>
+__device__ __forceinline__ void load_line(const real* u, const int st, real (&in)[P]) {
+#pragma unroll
+  for (int l = 0; l < P; ++l) in[l] = u[l * st];
+}
+template <int P, typename real>
+__device__ __forceinline__ void store_line(real* u, const int st, const real (&v)[P]) {
+#pragma unroll
+  for (int l = 0; l < P; ++l) u[l * st] = v[l];
+}
 
-// Element gradient into s.dQ (both kernels).  Requires s.Q (and s.Ja) filled and synchronized.
-template <int P, int EPB, typename real, bool AFFINE, bool IP, bool ST>
-__device__ __forceinline__ void element_gradient(const NSArgs<real>& a, NSTiles<P, EPB, real, AFFINE, ST>& s,
-                                                 const Phys<real>& ph, int le, int tid, int e, bool active,
-                                                 const real* geoE) {
-  constexpr int NP = P * P, FT = 4 * P;
-  const real* hatDT = s.mat;   // transposed: hatDT[l * P + i] = hatD(i, l)
-  const real* lb0 = s.mat + NP;
-  const real* lb1 = lb0 + P;
-  const real* lbw0 = lb1 + P;
-  const real* lbw1 = lbw0 + P;
-  const real* DT = lbw1 + P;   // transposed D
-  const int i = tid % P, j = tid / P;
-  if (!IP) {
-    // BR1 face terms u* dS n (outward normal of this element)
-    if (active) {
-      for (int t = tid; t < FT; t += NP) {
-        const int sd_ = t / P, kk = t % P;
-        const int4 sd = a.side[size_t(e) * 4 + sd_];
+// Shared memory of a CTA.  GRAD: the gradient kernel's (no RK register, no stored gradient to read).
+template <int P, int V, typename real, bool AFFINE, bool IP, bool AV, bool VISC, bool GRAD>
+struct NSTiles {
+  static constexpr int EPB = epb_ns_of(P, V), T = ns_threads(P, V);
+  static constexpr int NP = P * P, FT = 4 * P, PO = P | 1, NN = EPB * NP, NF = EPB * FT, GS = vol_geo_stride(P, AFFINE);
+  static constexpr int VM = sizeof(real) == 8 ? 16 : 32, V0 = EPB * P * PO;
+  static constexpr int VS = V0 + (VM + VM / 4 - V0 % VM) % VM;   // = VM / 4 modulo VM
+  static constexpr bool FACES = !(GRAD && IP);            // reads traces
+  static constexpr bool GT = (VISC && !GRAD) || (GRAD && !IP);   // 8-value records of the neighbours
+  // Side-node records as they are copied in (one thread each): strides of an odd number of 16-byte units, so that
+  // eight lanes' 128-bit reads fall into different banks.
+  static constexpr int RT = sizeof(real) == 8 ? 6 : 4, RG = sizeof(real) == 8 ? 10 : 12;
+  // Side tile of the fluxes (4 values) and gradient terms (8): variable-major, rows of PO per side, variable stride
+  // FS = VM / 4 modulo VM.
+  static constexpr int F0 = EPB * 4 * PO, FS = F0 + (VM + VM / 4 - F0 % VM) % VM;
+  static constexpr int FV = GRAD ? (IP ? (AFFINE ? 12 : 0) : 8) : (IP && VISC ? 12 : 4);
+  // The state record is needed again for the update; in double the Q tile holds the same values.
+  static constexpr bool KEEP_Q = sizeof(real) == 4 && !GRAD;
+  struct Once {                        // inputs of a group that are dead before its contraction (phase D): single,
+    double Q[KEEP_Q ? 2 : NN * 4];     // the next group's are fetched as soon as they are
+    real To[FACES ? NF * RT : 4];      // own traces
+    real Tn[FACES ? NF * RT : 4];      // neighbours' traces (or mortar fluxes)
+    real GTo[VISC && !GRAD ? NF * RG : 4];  // own gradient traces
+    real GTn[GT ? NF * RG : 4];        // neighbours' gradient traces (or mortar terms)
+    real dQ[!GRAD && !IP ? NN * 8 : 4];     // BR1 gradient
+    real sg[!AFFINE && FACES ? NF * 3 : 4];
+    double invh[EPB * 4], area[EPB * 4], mun[EPB * 4];
+  };
+  struct In {                          // inputs of a group that live longer: double
+    double Q[KEEP_Q ? NN * 4 : 2];
+    real vg[EPB * GS];
+    double mu[(EPB + 1) / 2 * 2];
+  };
+  alignas(16) Once one;
+  alignas(16) In in[2];
+  alignas(16) int4 side[3][EPB * 4];
+  real G[GRAD ? 4 : NN * 4];
+  // Q tile (interior penalty, indicator); Fc, Gc: derivatives along the lines, then contravariant fluxes, then
+  // their contractions
+  alignas(16) real Q[4 * VS];
+  real Fc[4 * VS], Gc[4 * VS];
+  real X[GRAD && !IP ? 4 * VS : 4], Y[GRAD && !IP ? 4 * VS : 4];   // BR1 volume terms of the second direction
+  real F[FV ? FV * FS : 4];
+  alignas(16) real sens[AV ? T / 32 * sensor_scratch(P) : 4];
+  unsigned long long mx[GRAD ? 1 : 4][GRAD ? 1 : T / 32];   // per-warp max |QDot| as bits (NaN above all)
+  static constexpr int REGS = sizeof(real) == 8 ? 128 : 80;
+  uint64_t bar[2];                     // inputs, RK register
+  __device__ __forceinline__ const double* state(int b) const { return KEEP_Q ? in[b].Q : one.Q; }
+};
+// CTAs per SM the launch bounds ask for: what shared memory holds, down to Tl::REGS registers a thread.  Left
+// to itself the compiler takes up to twice as many for the phase with the longest expressions.
+template <typename Tl>
+constexpr int ns_min_ctas() {
+  return cmax(1, cmin(cmin(int(227 * 1024 / (sizeof(Tl) + 1024)), 65536 / (Tl::T * Tl::REGS)), 32));
+}
+constexpr size_t MLP_BYTES = (size_t(MLP_PARAMS) * sizeof(float) + 15) / 16 * 16;   // after the tiles, when learned
+
+// The part of the persistent loop that both kernels share: barriers and prefetch.
+template <typename Tl, int P, typename real, bool AFFINE, bool IP, bool AV, bool VISC, bool GRAD>
+struct NSPipe {
+  static constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, GS = Tl::GS;
+  const NSArgs<real>& a;
+  Tl& s;
+  const int tid, n_groups;
+  unsigned phase = 0u;   // parities of the barriers
+
+  __device__ __forceinline__ int count(int g) const { return min(EPB, a.n_el - g * EPB); }
+  __device__ __forceinline__ void gave_up() const {
+    if (a.health) atomicOr(a.health, HEALTH_COPY);
+    if (a.health_host) *reinterpret_cast<volatile int*>(a.health_host) = 1;
+  }
+  // inputs of group g (those of struct In into half b), and the side table of the group after it (thread 0)
+  __device__ __forceinline__ void bulk(int g, int b, bool own_side, int slot) const {
+    constexpr unsigned R = sizeof(real);
+    const int e0 = g * EPB, n = count(g), gn = g + gridDim.x;
+    typename Tl::In& in = s.in[b];
+    uint64_t* bar = &s.bar[0];
+    const unsigned bq = n * NP * 32u;
+    const unsigned bd = !GRAD && !IP ? n * NP * 8u * R : 0u, bv = n * GS * R, bs = !AFFINE && Tl::FACES ? n * FT * 3u * R : 0u;
+    const unsigned bh = IP && VISC && !GRAD ? n * 32u : 0u, ba = AV && !GRAD ? n * 32u : 0u;
+    const unsigned b0 = own_side ? n * 64u : 0u, bn = gn < n_groups ? count(gn) * 64u : 0u;
+    mbar_expect(bar, bq + bd + bv + bs + bh + ba + b0 + bn);
+    bulk_copy(const_cast<double*>(s.state(b)), a.Q + size_t(e0) * NP * 4, bq, bar);
+    if (b0) bulk_copy(s.side[slot], a.side + size_t(e0) * 4, b0, bar);
+    if (bd) bulk_copy(s.one.dQ, a.dQ + size_t(e0) * NP * 8, bd, bar);
+    bulk_copy(in.vg, a.vol_geo + size_t(e0) * GS, bv, bar);
+    if (bs) bulk_copy(s.one.sg, a.side_geo + size_t(e0) * FT * 3, bs, bar);
+    if (bh) bulk_copy(s.one.invh, a.side_invh + size_t(e0) * 4, bh, bar);
+    if (ba) bulk_copy(s.one.area, a.side_area + size_t(e0) * 4, ba, bar);
+    if (bn) bulk_copy(s.side[slot == 2 ? 0 : slot + 1], a.side + size_t(gn) * EPB * 4, bn, bar);
+  }
+  // the side-node records of group g, each copied and read by one thread; the viscosities of the group's elements
+  // (into half b) and of their neighbours
+  __device__ __forceinline__ void rows(int g, int b, const int4* side) const {
+    constexpr int RT = Tl::RT, RG = Tl::RG;
+    typename Tl::Once& one = s.one;
+    const int n = count(g);
+    if (Tl::FACES)
+      for (int x = tid; x < n * FT; x += T) {
+        const int t = x % FT, kk = t % P;
+        const int4 sd = side[(x / FT) * 4 + t / P];
         const int kind = sd.y & 15;
-        if (kind == SIDE_FLUX) {   // p-nonconforming or subdivided edge: terms from the mortar kernel
-          const real* gp = a.NFG + (size_t(sd.x) * P + kk) * 8;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) s.face[k][le][t] = gp[k];
-          continue;
+        const size_t own = size_t(g) * EPB * FT + x;
+        if (kind != SIDE_FLUX) {
+          cp_async_4(&one.To[x * RT], a.T_in + own * 4);
+          if (VISC && !GRAD) {
+            cp_async_4(&one.GTo[x * RG], a.GT + own * 8);
+            cp_async_4(&one.GTo[x * RG + 4], a.GT + own * 8 + 4);
+          }
         }
-        const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-        real qo[4];
-        trace4<P, EPB, real>(s.Q, le, sd_, kk, lbv, qo);
-        const real* g3 = AFFINE ? a.side_geo + (size_t(e) * 4 + sd_) * 3 : a.side_geo + ((size_t(e) * 4 + sd_) * P + kk) * 3;
-        const real nx = real(g3[0]), ny = real(g3[1]), dS = real(g3[2]);
-        real us[4];
         if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
-          const int kn = (sd.y & SIDE_REVERSED) ? (P - 1 - kk) : kk;
-          real tp[4];
-          ld4(a.T_in + (size_t(sd.x) * P + kn) * 4, tp);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) us[k] = kind == SIDE_RIGHT ? real(0.5) * (tp[k] + qo[k]) : real(0.5) * (qo[k] + tp[k]);
-        } else {
-          real uB[4];
-          bc_states(ph, a.zones[sd.z], qo, nx, ny, uB, us, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
-        }
-        const real sg = kind == SIDE_RIGHT ? real(-1) : real(1);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          s.face[k][le][t] = (sg * us[k]) * dS * nx;
-          s.face[4 + k][le][t] = (sg * us[k]) * dS * ny;
+          const size_t row = size_t(sd.x) * P + ((sd.y & SIDE_REVERSED) ? P - 1 - kk : kk);
+          cp_async_4(&one.Tn[x * RT], a.T_in + row * 4);
+          if (VISC && !GRAD) {
+            cp_async_4(&one.GTn[x * RG], a.GT + row * 8);
+            cp_async_4(&one.GTn[x * RG + 4], a.GT + row * 8 + 4);
+          }
+        } else if (kind == SIDE_FLUX) {
+          const size_t row = size_t(sd.x) * P + kk;
+          if (!GRAD) cp_async_4(&one.Tn[x * RT], a.NF + row * 4);
+          if (GRAD ? !IP : (VISC && IP && a.grad_faces)) {
+            cp_async_4(&one.GTn[x * RG], a.NFG + row * 8);
+            cp_async_4(&one.GTn[x * RG + 4], a.NFG + row * 8 + 4);
+          }
         }
       }
+    if (AV && !GRAD) {
+      for (int x = tid; x < n * 4; x += T) {
+        const int4 sd = side[x];
+        const int kind = sd.y & 15;
+        const bool inner = (kind == SIDE_LEFT || kind == SIDE_RIGHT) && sd.z < 0;
+        cp_async_real(&one.mun[x], a.mu_av + (inner ? sd.x >> 2 : g * EPB + x / 4));
+      }
+      for (int x = tid; x < n; x += T) cp_async_real(&s.in[b].mu[x], a.mu_av + g * EPB + x);
+    }
+    cp_async_commit();
+  }
+  __device__ __forceinline__ void start() const {
+    if (tid == 0) {
+      for (int k = 0; k < 2; ++k) mbar_init(&s.bar[k]);
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      bulk(blockIdx.x, 0, true, 0);
+    }
+    rows(blockIdx.x, 0, a.side + size_t(blockIdx.x) * EPB * 4);
+    __syncthreads();   // the barriers are initialised
+  }
+  __device__ __forceinline__ void wait(int k) {
+    if (!mbar_wait(&s.bar[k], (phase >> k) & 1u)) gave_up();
+    phase ^= 1u << k;
+  }
+  // top of the loop for group g: its inputs are there, every thread is done with the group before, and its RK
+  // register is on its way
+  __device__ __forceinline__ void next(int g, bool rk) {
+    wait(0);
+    cp_async_wait_all();
+    __syncthreads();
+    if (rk && tid == 0) {
+      const unsigned bytes = count(g) * NP * 4u * unsigned(sizeof(real));
+      mbar_expect(&s.bar[1], bytes);
+      bulk_copy(s.G, a.G + size_t(g) * EPB * NP * 4, bytes, &s.bar[1]);
+    }
+  }
+  // after the barrier behind the face tasks: the next group's records
+  __device__ __forceinline__ void prefetch_rows(int g, int b, int next_slot) const {
+    if (g + int(gridDim.x) < n_groups) rows(g + gridDim.x, b ^ 1, s.side[next_slot]);
+  }
+  // after the barrier behind the last use of struct Once: the rest of the next group's inputs
+  __device__ __forceinline__ void prefetch(int g, int b, int next_slot) const {
+    if (tid == 0 && g + int(gridDim.x) < n_groups) bulk(g + gridDim.x, b ^ 1, false, next_slot);
+  }
+};
+
+// Derivatives D u along the lines of the Q tile into Fc (xi) and Gc (eta), n_act elements.
+template <int P, typename Tl, typename real>
+__device__ __forceinline__ void tile_derivatives(Tl& s, const real* D, int n_act, int tid) {
+  constexpr int EPB = Tl::EPB, VS = Tl::VS, PO = Tl::PO, NF = Tl::NF;
+  for (int x = tid; x < 2 * NF; x += Tl::T) {   // x = (direction, variable, element, line)
+    const int y = x % NF, v = y / (P * EPB), le = (y / P) % EPB, m = y % P;
+    if (le >= n_act) continue;
+    real in[P], out[P];
+    if (x < NF) {
+      const int o = v * VS + (le * P + m) * PO;
+      load_line<P>(&s.Q[o], 1, in);
+      apply<P>(D, in, out);
+      store_line<P>(&s.Fc[o], 1, out);
+    } else {
+      const int o = v * VS + le * P * PO + m;
+      load_line<P>(&s.Q[o], PO, in);
+      apply<P>(D, in, out);
+      store_line<P>(&s.Gc[o], PO, out);
+    }
+  }
+}
+
+// Cartesian gradient of node m (element le) from the derivative tiles.
+template <int P, typename Tl, bool AFFINE, typename real>
+__device__ __forceinline__ void node_gradient(const Tl& s, const real* gp, int o, real* gx, real* gy) {
+  const real Ja00 = gp[0], Ja01 = gp[1], Ja10 = gp[2], Ja11 = gp[3], iJ = gp[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const real dxi = s.Fc[k * Tl::VS + o], deta = s.Gc[k * Tl::VS + o];
+    gx[k] = (dxi * Ja00 + deta * Ja01) * iJ;
+    gy[k] = (dxi * Ja10 + deta * Ja11) * iJ;
+  }
+}
+
+// The traces at both ends of every line of tile U (4 variables) into rec[x * R + v] in global memory (x the
+// element's side node), the variable fastest over the lanes.
+template <int P, int R, bool REL, typename Tl, typename real>
+__device__ __forceinline__ void tile_traces(const real* U, const real* c0, const real* c1, real* rec, int n_act, int tid) {
+  constexpr int VS = Tl::VS, PO = Tl::PO, FT = Tl::FT;
+  for (int x = tid; x < n_act * FT; x += Tl::T) {   // x = (element, line, variable)
+    const int v = x & 3, le = x / FT, m = (x >> 2) % P;
+    real* r = rec + size_t(le) * FT * R + v;
+    real in[P];
+    load_line<P>(U + v * VS + (le * P + m) * PO, 1, in);
+    r[(3 * P + m) * R] = REL ? trace_dot<P>(c0, in) : dot<P>(c0, in);
+    r[(P + m) * R] = REL ? trace_dot<P>(c1, in) : dot<P>(c1, in);
+    load_line<P>(U + v * VS + le * P * PO + m, PO, in);
+    r[m * R] = REL ? trace_dot<P>(c0, in) : dot<P>(c0, in);
+    r[(2 * P + m) * R] = REL ? trace_dot<P>(c1, in) : dot<P>(c1, in);
+  }
+}
+
+// Gradient traces of the state in the Q tile (element-local gradient) into GT.  Affine elements: straight from
+// the state -- along a side, D applied to the side's Q traces; across it, each normal line of nodes contracted
+// with lb^T D -- the same as the nodal gradient interpolated to the side, without forming it at every node.
+// The Q traces go to T_out when given.  Starts after a barrier on the Q tile; uses the side tile (affine) or Fc and
+// Gc (curved).
+template <int P, bool AFFINE, typename Tl, typename real>
+__device__ __forceinline__ void gradient_traces(Tl& s, const NSOps<P, real>& op, const real* vg, real* T_out, real* GT,
+                                                int n_act, int tid) {
+  constexpr int VS = Tl::VS, PO = Tl::PO, FT = Tl::FT, NP = Tl::NP, GS = Tl::GS, FS = Tl::FS;
+  if constexpr (AFFINE) {
+    for (int x = tid; x < n_act * FT; x += Tl::T) {   // x = (element, line, variable)
+      const int v = x & 3, le = x / FT, m = (x >> 2) % P;
+      const auto end = [&](int side, real t, real d) {   // trace and normal derivative
+        const int y = v * FS + (le * 4 + side) * PO + m;
+        s.F[y] = t;
+        s.F[4 * FS + y] = d;
+        if (T_out) T_out[size_t(le * FT + side * P + m) * 4 + v] = t;
+      };
+      real in[P];
+      load_line<P>(&s.Q[v * VS + (le * P + m) * PO], 1, in);
+      end(3, dot<P>(op.lb0, in), dot<P>(op.dl0, in));
+      end(1, dot<P>(op.lb1, in), dot<P>(op.dl1, in));
+      load_line<P>(&s.Q[v * VS + le * P * PO + m], PO, in);
+      end(0, dot<P>(op.lb0, in), dot<P>(op.dl0, in));
+      end(2, dot<P>(op.lb1, in), dot<P>(op.dl1, in));
     }
     __syncthreads();
-  }
-  if (active) {
-    real Ja00, Ja01, Ja10, Ja11, iJ;
-    if constexpr (AFFINE) { Ja00 = geoE[0]; Ja01 = geoE[1]; Ja10 = geoE[2]; Ja11 = geoE[3]; iJ = geoE[4]; }
-    else { Ja00 = s.Ja[0][le][tid]; Ja01 = s.Ja[1][le][tid]; Ja10 = s.Ja[2][le][tid]; Ja11 = s.Ja[3][le][tid];
-           iJ = real(1) / s.Ja[4][le][tid]; }
-    // the operator rows and metrics of a node are loaded once per l and reused for the 4 variables
-    if (IP) {
-      real dxi[4] = {real(0), real(0), real(0), real(0)}, deta[4] = {real(0), real(0), real(0), real(0)};
+    for (int x = tid; x < n_act * 16; x += Tl::T) {   // x = (element, side, variable)
+      const int v = x & 3, sd = (x >> 2) & 3, le = x >> 4, y = v * FS + (le * 4 + sd) * PO;
+      const real* gp = vg + le * GS;
+      const real Ja00 = gp[0], Ja01 = gp[1], Ja10 = gp[2], Ja11 = gp[3], iJ = gp[4];
+      real in[P], dt[P];
+      load_line<P>(&s.F[y], 1, in);
+      apply<P>(op.D, in, dt);
+      const bool alongXi = (sd & 1) == 0;   // bottom / top: along the side is xi; right / left: eta
 #pragma unroll
-      for (int l = 0; l < P; ++l) {
-        const real di = DT[l * P + i], dj = DT[l * P + j];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          dxi[k] += di * s.Q[k][le][j * P + l];
-          deta[k] += dj * s.Q[k][le][l * P + i];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        s.dQ[0][k][le][tid] = (dxi[k] * Ja00 + deta[k] * Ja01) * iJ;
-        s.dQ[1][k][le][tid] = (dxi[k] * Ja10 + deta[k] * Ja11) * iJ;
-      }
-    } else {
-      real v0[4] = {real(0), real(0), real(0), real(0)}, v1[4] = {real(0), real(0), real(0), real(0)};
-      if constexpr (AFFINE) {
-        real axi[4] = {real(0), real(0), real(0), real(0)}, aeta[4] = {real(0), real(0), real(0), real(0)};
-#pragma unroll
-        for (int l = 0; l < P; ++l) {
-          const real hi = hatDT[l * P + i], hj = hatDT[l * P + j];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            axi[k] += hi * s.Q[k][le][j * P + l];
-            aeta[k] += hj * s.Q[k][le][l * P + i];
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          v0[k] = axi[k] * Ja00 + aeta[k] * Ja01;
-          v1[k] = axi[k] * Ja10 + aeta[k] * Ja11;
-        }
-      } else {
-#pragma unroll
-        for (int l = 0; l < P; ++l) {
-          const int nx_ = j * P + l, ny_ = l * P + i;
-          const real hi = hatDT[l * P + i], hj = hatDT[l * P + j];
-          const real j0 = s.Ja[0][le][nx_], j1 = s.Ja[1][le][ny_], j2 = s.Ja[2][le][nx_], j3 = s.Ja[3][le][ny_];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const real qx = s.Q[k][le][nx_] * hi, qy = s.Q[k][le][ny_] * hj;
-            v0[k] += qx * j0 + qy * j1;
-            v1[k] += qx * j2 + qy * j3;
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const real l0 = s.face[k][le][0 * P + i] * lbw0[j] + s.face[k][le][1 * P + j] * lbw1[i] +
-                        s.face[k][le][2 * P + i] * lbw1[j] + s.face[k][le][3 * P + j] * lbw0[i];
-        const real l1 = s.face[4 + k][le][0 * P + i] * lbw0[j] + s.face[4 + k][le][1 * P + j] * lbw1[i] +
-                        s.face[4 + k][le][2 * P + i] * lbw1[j] + s.face[4 + k][le][3 * P + j] * lbw0[i];
-        s.dQ[0][k][le][tid] = (-v0[k] + l0) * iJ;
-        s.dQ[1][k][le][tid] = (-v1[k] + l1) * iJ;
+      for (int k = 0; k < P; ++k) {
+        const real d = s.F[4 * FS + y + k];
+        const real dxi = alongXi ? dt[k] : d, deta = alongXi ? d : dt[k];
+        real* g = GT + size_t(le * FT + sd * P + k) * 8 + v;
+        g[0] = (dxi * Ja00 + deta * Ja01) * iJ;
+        g[4] = (dxi * Ja10 + deta * Ja11) * iJ;
       }
     }
+  } else {
+    if (T_out) tile_traces<P, 4, false, Tl>(s.Q, op.lb0, op.lb1, T_out, n_act, tid);
+    tile_derivatives<P>(s, op.D, n_act, tid);
+    __syncthreads();
+    for (int m = tid; m < n_act * NP; m += Tl::T) {
+      const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
+      real gx[4], gy[4];
+      node_gradient<P, Tl, AFFINE>(s, vg + le * GS + node * 5, o, gx, gy);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) { s.Fc[k * VS + o] = gx[k]; s.Gc[k * VS + o] = gy[k]; }
+    }
+    __syncthreads();
+    tile_traces<P, 8, false, Tl>(s.Fc, op.lb0, op.lb1, GT, n_act, tid);
+    tile_traces<P, 8, false, Tl>(s.Gc, op.lb0, op.lb1, GT + 4, n_act, tid);
   }
 }
 
-template <int P, int EPB, typename real, bool AFFINE, bool ST>
-__device__ __forceinline__ void load_tiles(const NSArgs<real>& a, NSTiles<P, EPB, real, AFFINE, ST>& s, int flat, int le,
-                                           int tid, int e, bool active, real* geoE) {
-  constexpr int NP = P * P;
-  // hatD and D are held transposed (column l contiguous): a warp then reads hatD(i, l) over its nodes'
-  // i from consecutive words instead of a stride of P (bank conflicts)
-  for (int k = flat; k < 3 * NP + 7 * P; k += blockDim.x) {
-    int src = k;
-    if (k < NP) src = (k % P) * P + k / P;
-    else if (k >= NP + 4 * P && k < 2 * NP + 4 * P) { const int m = k - NP - 4 * P; src = NP + 4 * P + (m % P) * P + m / P; }
-    s.mat[k] = real(a.mats[src]);
-  }
-  if (active) {
-    const double2* qp = reinterpret_cast<const double2*>(a.Q + (size_t(e) * NP + tid) * 4);
-    const double2 q01 = qp[0], q23 = qp[1];
-    s.Q[0][le][tid] = real(q01.x); s.Q[1][le][tid] = real(q01.y);
-    s.Q[2][le][tid] = real(q23.x); s.Q[3][le][tid] = real(q23.y);
-    if constexpr (AFFINE) {
-#pragma unroll
-      for (int k = 0; k < 5; ++k) geoE[k] = a.vol_geo[size_t(e) * vol_geo_stride(P, true) + k];
-    } else {
-      const real* gp = a.vol_geo + size_t(e) * vol_geo_stride(P, false) + tid * 5;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) s.Ja[k][le][tid] = real(gp[k]);
-      s.Ja[4][le][tid] = real(a.jac[size_t(e) * NP + tid]);
-      geoE[4] = real(gp[4]);
-    }
-  }
-}
-
-// JumpsBasedElementViscosity (Approximation/DGArtificialDissipation.f90:277-338) of each element of the
-// CTA into a.mu_av.  Edge jumps (Edge_ComputeJumps and the boundary/curved variants,
+// JumpsBasedElementViscosity (Approximation/DGArtificialDissipation.f90:277-338) of each element into a.mu_av,
+// one thread per side node.  Edge jumps (Edge_ComputeJumps and the boundary/curved variants,
 // Mesh/QuadElement_EdgeProcedures.incf:1348-1619): sum over the edge nodes, in the edge's order, of
 // w (2 (QL-QR)/(QL+QR))^2 dS for rho and rhoE; boundary and periodic edges use the viscous boundary
-// state (uSB) and dS at their first node.  Uses s.face[0..1] as scratch; ends with a barrier.
-template <int P, int EPB, typename real, bool AFFINE, bool ST>
-__device__ __forceinline__ void element_viscosity(const NSArgs<real>& a, NSTiles<P, EPB, real, AFFINE, ST>& s,
-                                                  const Phys<real>& ph, int le, int tid, int e, bool active) {
-  constexpr int NP = P * P, FT = 4 * P;
-  if (a.sensor.kind != SENSOR_JUMPS) {   // modal-decay or learned indicator (hg_sensor.cuh)
-    // evaluated on the first stage of a time step (and for a bare time derivative); the later stages
-    // of the step keep that viscosity.  The reference's jumps indicator is re-evaluated every stage.
-    if (!a.first) return;
-    const int n_active = a.n_el - int(blockIdx.x) * EPB < EPB ? a.n_el - int(blockIdx.x) * EPB : EPB;
-    const SensorOut so = element_sensor<P, EPB, real>(a.sensor, ph, s.Q, n_active, s.mat + 2 * NP + 7 * P, le,
-                                                      tid, active, nullptr);
-    if (active && tid == 0) a.mu_av[e] = a.av_el[2 * size_t(e)] * so.g;
-    __syncthreads();
-    return;
+// state (uSB) and dS at their first node.  Reads traces only (the elements' own are in T_in too): bound by
+// their loads.
+template <int P, typename real>
+struct EdgeWeights { real w[P]; };
+__host__ __device__ constexpr int jumps_epb(int P) { return 128 / (4 * P); }
+template <int P, typename real, bool AFFINE>
+__global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSArgs<real> a,
+                                                    const __grid_constant__ EdgeWeights<P, real> ew) {
+  constexpr int FT = 4 * P, EPB = jumps_epb(P);
+  __shared__ real jr_[EPB * FT], je_[EPB * FT];
+  __shared__ real s_w[P];
+  const int tid = threadIdx.x, e0 = blockIdx.x * EPB, n_act = min(EPB, a.n_el - e0);
+  if (tid < P) {
+    real w = ew.w[0];
+#pragma unroll
+    for (int k = 1; k < P; ++k) w = tid == k ? ew.w[k] : w;
+    s_w[tid] = w;
   }
-  const real* lb0 = s.mat + NP;
-  const real* lb1 = lb0 + P;
-  const real* wq = s.mat + 2 * NP + 6 * P;
-  if (active) {
-    for (int t = tid; t < FT; t += NP) {
-      const int sd_ = t / P, kk = t % P;
-      const int4 sd = a.side[size_t(e) * 4 + sd_];
-      const int kind = sd.y & 15;
-      if (kind == SIDE_FLUX) {   // edge between orders or subdivided edge: the mortar kernel's jump sums
-        s.face[0][le][t] = kk == 0 ? a.NJ[size_t(sd.x) * 2] : real(0);
-        s.face[1][le][t] = kk == 0 ? a.NJ[size_t(sd.x) * 2 + 1] : real(0);
-        continue;
-      }
-      const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-      real qo[4];
-      trace4<P, EPB, real>(s.Q, le, sd_, kk, lbv, qo);
-      const size_t sbase = size_t(e) * 4 + sd_;
-      real qn0, qn3;
+  Phys<real> ph;
+  ph.load(a.pc);
+  __syncthreads();
+  if (tid < n_act * FT) {
+    const int sd_ = (tid % FT) / P, kk = tid % P;
+    const size_t sbase = size_t(e0) * 4 + tid / P, slot = size_t(e0) * FT + tid;
+    const int4 sd = a.side[sbase];
+    const int kind = sd.y & 15;
+    if (kind == SIDE_FLUX) {   // edge between orders or subdivided edge: the mortar kernel's jump sums
+      jr_[tid] = kk == 0 ? a.NJ[size_t(sd.x) * 2] : real(0);
+      je_[tid] = kk == 0 ? a.NJ[size_t(sd.x) * 2 + 1] : real(0);
+    } else {
+      real qo[4], qn0, qn3;
+      ld4(a.T_in + slot * 4, qo);
       bool node0 = true;
       if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
         const int kn = (sd.y & SIDE_REVERSED) ? (P - 1 - kk) : kk;
-        const real* tp = a.T_in + (size_t(sd.x) * P + kn) * 4;
-        qn0 = tp[0];
-        qn3 = tp[3];
+        real qn[4];
+        ld4(a.T_in + (size_t(sd.x) * P + kn) * 4, qn);
+        qn0 = qn[0];
+        qn3 = qn[3];
         node0 = sd.z >= 0;   // periodic edges are boundary edges of the reference
       } else {
-        const real* g3 = AFFINE ? a.side_geo + sbase * 3 : a.side_geo + (sbase * P + kk) * 3;
+        const real* g3 = AFFINE ? a.side_geo + sbase * 3 : a.side_geo + slot * 3;
         real uB[4], uS[4];
-        bc_states(ph, a.zones[sd.z], qo, real(g3[0]), real(g3[1]), uB, uS,
-                  sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
+        bc_states(ph, a.zones[sd.z], qo, g3[0], g3[1], uB, uS, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
         qn0 = uS[0];
         qn3 = uS[3];
       }
-      const real dSn = real(AFFINE ? a.side_geo[sbase * 3 + 2] : a.side_geo[(sbase * P + (node0 ? 0 : kk)) * 3 + 2]);
+      const real dSn = AFFINE ? a.side_geo[sbase * 3 + 2] : a.side_geo[(sbase * P + (node0 ? 0 : kk)) * 3 + 2];
       const real jr = real(2) * (qo[0] - qn0) / (qo[0] + qn0);
       const real je = real(2) * (qo[3] - qn3) / (qo[3] + qn3);
-      s.face[0][le][t] = wq[kk] * jr * jr * dSn;
-      s.face[1][le][t] = wq[kk] * je * je * dSn;
+      jr_[tid] = s_w[kk] * jr * jr * dSn;
+      je_[tid] = s_w[kk] * je * je * dSn;
     }
+    (void)sd_;
   }
   __syncthreads();
-  if (active && tid == 0) {
+  if (tid < n_act) {
+    const int e = e0 + tid;
     real gr = real(0), ge = real(0);
 #pragma unroll
     for (int sd_ = 0; sd_ < 4; ++sd_) {
@@ -349,9 +486,9 @@ __device__ __forceinline__ void element_viscosity(const NSArgs<real>& a, NSTiles
       const bool rev = (fl & 15) == SIDE_RIGHT && (fl & SIDE_REVERSED);
       real sr = real(0), se = real(0);
       for (int n = 0; n < P; ++n) {
-        const int kk = rev ? (P - 1 - n) : n;
-        sr = sr + s.face[0][le][sd_ * P + kk];
-        se = se + s.face[1][le][sd_ * P + kk];
+        const int kk = tid * FT + sd_ * P + (rev ? (P - 1 - n) : n);
+        sr = sr + jr_[kk];
+        se = se + je_[kk];
       }
       gr = gr + sr;
       ge = ge + se;
@@ -368,567 +505,552 @@ __device__ __forceinline__ void element_viscosity(const NSArgs<real>& a, NSTiles
   }
 }
 
-template <int P, int EPB, typename real, bool AFFINE, bool IP, bool AV>
-__global__ void __launch_bounds__(block_of(P, EPB)) ns_gradient_kernel(NSArgs<real> a) {
-  constexpr int NP = P * P, FT = 4 * P;
-  __shared__ NSTiles<P, EPB, real, AFFINE, false> s;
-  const int flat = threadIdx.x, le = flat / NP, tid = flat - le * NP;
-  const int e = blockIdx.x * EPB + le;
-  const bool active = le < EPB && e < a.n_el;
+// Gradient kernel.  BR1: lifted gradient (stored) and its traces; interior penalty: gradient traces of the
+// resident state.  Then the modal or learned indicator, on the first stage of a time step (and for a bare
+// time derivative); the later stages of the step keep that viscosity.
+template <int P, int V, typename real, bool AFFINE, bool IP, bool AV>
+__global__ void __launch_bounds__(ns_threads(P, V))
+    ns_gradient_kernel(const __grid_constant__ NSArgs<real> a, const __grid_constant__ NSOps<P, real> op) {
+  using Tl = NSTiles<P, V, real, AFFINE, IP, AV, true, true>;
+  constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, PO = Tl::PO, VS = Tl::VS, GS = Tl::GS, NF = Tl::NF,
+                FS = Tl::FS, RT = Tl::RT, RG = Tl::RG;
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  Tl& s = *reinterpret_cast<Tl*>(stage_smem);
+  float* s_w = reinterpret_cast<float*>(stage_smem + sizeof(Tl));
+  const int tid = threadIdx.x, n_groups = (a.n_el + EPB - 1) / EPB;
+  NSPipe<Tl, P, real, AFFINE, IP, AV, true, true> pipe{a, s, tid, n_groups};
   Phys<real> ph;
   ph.load(a.pc);
-  real geoE[5];
-  load_tiles(a, s, flat, le, tid, e, active, geoE);
-  __syncthreads();
-  // the interior-penalty gradient is element-local: without viscous fluxes nothing here uses it (the
-  // launch then only evaluates the indicator); a.viscous is uniform over the launch
-  if (!IP || a.viscous) {
-    element_gradient<P, EPB, real, AFFINE, IP>(a, s, ph, le, tid, e, active, geoE);
-    __syncthreads();
-  }
-  if (AV) element_viscosity<P, EPB, real, AFFINE>(a, s, ph, le, tid, e, active);
-  if (!active) return;
-  if (!IP) {   // the lifted gradient is not local: store it for the stage kernel
-    real* g = a.dQ + size_t(e) * 8 * NP + tid;
+  const bool sense = AV && a.sensor.kind != SENSOR_JUMPS && a.first;
+  if (sense && a.sensor.kind == SENSOR_LEARNED) sensor_weights_async(s_w, a.sensor.mlp, tid, T);
+  pipe.start();
+  FlatG flat_g;
+  int b = 0, slot = 0;
+  for (int g = blockIdx.x; g < n_groups; g += gridDim.x) {
+    const int e0 = g * EPB, n_act = pipe.count(g), next_slot = slot == 2 ? 0 : slot + 1;
+    pipe.next(g, false);
+    typename Tl::In& in = s.in[b];
+    const int4* side = s.side[slot];
+    const double* Qg = s.state(b);
+    // In float the BR1 gradient is formed from the state minus the element's first node (exactly representable,
+    // subtracted in double): the lifted gradient of a constant vanishes, and the 24-bit rounding of the
+    // state itself and of its contraction -- the largest error of a float time derivative otherwise -- is
+    // taken of the variation instead.  (Not where the indicator reads the tile afterwards, nor in elements
+    // with a mortar side, whose terms hold the whole state.)
+    const auto shift = [&](int le) {
+      bool on = sizeof(real) == 4 && !IP && !sense;
+      if (on && a.NFG)
+        for (int k = 0; k < 4; ++k) on = on && (side[le * 4 + k].y & 15) != SIDE_FLUX;
+      return on;
+    };
+    for (int m = tid; m < n_act * NP; m += T) {
+      const int o = (m / P) * PO + m % P;
+      double q[4];
+      ld4(Qg + m * 4, q);
+      const bool sh = shift(m / NP);
 #pragma unroll
-    for (int d = 0; d < 2; ++d)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) g[(d * 4 + k) * NP] = s.dQ[d][k][le][tid];
-  }
-  if (!a.viscous) return;   // gradient traces only feed viscous face fluxes
-  const real* lb0 = s.mat + NP;
-  const real* lb1 = lb0 + P;
-  for (int t = tid; t < FT; t += NP) {
-    const int sd_ = t / P, kk = t % P;
-    const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-    real* gp = a.GT + ((size_t(e) * 4 + sd_) * P + kk) * 8;
-    real tx[4], ty[4];
-    trace4<P, EPB, real>(s.dQ[0], le, sd_, kk, lbv, tx);
-    trace4<P, EPB, real>(s.dQ[1], le, sd_, kk, lbv, ty);
-    st4(gp, tx);
-    st4(gp + 4, ty);
-  }
-}
-
-// Volume flux of node n of element le: F = Fi - (mu + mu_a) Fv (- mu_a grad Q for the Laplacian
-// dissipation), contravariant, into s.Fc and s.Gc (QDotVolumeLoop, DGSpatialDiscretizationMethods.f90:
-// 243-268).  Reads the node's Q and gradient from the tiles.
-template <int P, int EPB, typename real, bool AFFINE, bool IP, bool AV>
-__device__ __forceinline__ void ns_volume_flux(const NSArgs<real>& a, NSTiles<P, EPB, real, AFFINE>& s,
-                                               const Phys<real>& ph, int le, int n, real mu_e, bool need_grad,
-                                               bool visc, const real* geoE) {
-  constexpr int NP = P * P;
-  const int i = n % P, j = n / P;
-  const real mu = ph.mu;
-  real Ja00, Ja01, Ja10, Ja11;
-  if constexpr (AFFINE) { Ja00 = geoE[0]; Ja01 = geoE[1]; Ja10 = geoE[2]; Ja11 = geoE[3]; }
-  else { Ja00 = s.Ja[0][le][n]; Ja01 = s.Ja[1][le][n]; Ja10 = s.Ja[2][le][n]; Ja11 = s.Ja[3][le][n]; }
-  real q[4], gx[4], gy[4], fi[4], gi[4], fv[4], gv[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) { q[k] = s.Q[k][le][n]; gx[k] = s.dQ[0][k][le][n]; gy[k] = s.dQ[1][k][le][n]; }
-  inviscid_flux(ph, q, fi, gi);
-  if (visc) viscous_flux(ph, q, gx, gy, fv, gv);
-  else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) { fv[k] = real(0); gv[k] = real(0); }
-  }
-  const real mu_v = (AV && a.av == 2) ? mu + mu_e : mu;
-  real ax[4] = {real(0), real(0), real(0), real(0)}, ay[4] = {real(0), real(0), real(0), real(0)};
-  if (AV && a.av == 1 && need_grad) {   // Laplacian: mu_e times the element-local gradient (ComputeInteriorGradient)
-    if (IP) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { ax[k] = gx[k]; ay[k] = gy[k]; }
+      for (int k = 0; k < 4; ++k) s.Q[k * VS + o] = real(sh ? q[k] - double(real(Qg[(m / NP) * NP * 4 + k])) : q[k]);
+    }
+    if constexpr (IP) {
+      __syncthreads();
+      pipe.prefetch(g, b, next_slot);
+      if (a.viscous) {
+        gradient_traces<P, AFFINE>(s, op, in.vg, static_cast<real*>(nullptr), a.GT + size_t(e0) * FT * 8, n_act, tid);
+      }
     } else {
-      const real* DT = s.mat + NP + 4 * P;   // D (transposed) follows hatD, lb0, lb1, lbw0, lbw1
-      const real iJl = AFFINE ? geoE[4] : real(1) / s.Ja[4][le][n];
+      // face terms u* dS n (outward normal of this element)
+      for (int x = tid; x < n_act * FT; x += T) {
+        const int t = x % FT, sd_ = t / P, kk = t % P, le = x / FT;
+        const int4 sd = side[le * 4 + sd_];
+        const int kind = sd.y & 15;
+        const int y = (le * 4 + sd_) * PO + kk;
+        if (kind == SIDE_FLUX) {   // the mortar kernel's terms
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        real dxi = real(0), deta = real(0);
-#pragma unroll
-        for (int l = 0; l < P; ++l) {
-          dxi += DT[l * P + i] * s.Q[k][le][j * P + l];
-          deta += DT[l * P + j] * s.Q[k][le][l * P + i];
+          for (int k = 0; k < 8; ++k) s.F[k * FS + y] = s.one.GTn[x * RG + k];
+          continue;
         }
-        ax[k] = (dxi * Ja00 + deta * Ja01) * iJl;
-        ay[k] = (dxi * Ja10 + deta * Ja11) * iJl;
+        real qo[4], us[4], c[4];
+        ld4(&s.one.To[x * RT], qo);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] = shift(le) ? real(Qg[le * NP * 4 + k]) : real(0);
+        const real* g3 = AFFINE ? &in.vg[le * GS + 8 + sd_ * 3] : &s.one.sg[x * 3];
+        const real nx = g3[0], ny = g3[1], dS = g3[2];
+        if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
+          real tp[4];
+          ld4(&s.one.Tn[x * RT], tp);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) us[k] = real(0.5) * ((tp[k] - c[k]) + (qo[k] - c[k]));
+        } else {
+          real uB[4];
+          bc_states(ph, a.zones[sd.z], qo, nx, ny, uB, us, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) us[k] -= c[k];
+        }
+        const real sg = kind == SIDE_RIGHT ? -dS : dS;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s.F[k * FS + y] = us[k] * sg * nx;
+          s.F[(4 + k) * FS + y] = us[k] * sg * ny;
+        }
+      }
+      __syncthreads();
+      pipe.prefetch(g, b, next_slot);
+      pipe.prefetch_rows(g, b, next_slot);
+      // per line: minus the volume term plus the lift at its ends, for the x and y components; rows into Fc, Gc,
+      // columns into X, Y
+      for (int x = tid; x < 2 * NF; x += T) {   // x = (direction, variable, element, line)
+        const int y = x % NF, v = y / (P * EPB), le = (y / P) % EPB, m = y % P;
+        if (le >= n_act) continue;
+        const bool xi = x < NF;
+        const int o = xi ? v * VS + (le * P + m) * PO : v * VS + le * P * PO + m, st = xi ? 1 : PO;
+        const real* f0 = &s.F[v * FS + (le * 4 + (xi ? 3 : 0)) * PO + m];
+        const real* f1 = &s.F[v * FS + (le * 4 + (xi ? 1 : 2)) * PO + m];
+        real q[P], ox[P], oy[P];
+#pragma unroll
+        for (int l = 0; l < P; ++l) q[l] = s.Q[o + l * st];
+        if constexpr (AFFINE) {
+          const real* gp = &in.vg[le * GS];
+          const real jx = xi ? gp[0] : gp[1], jy = xi ? gp[2] : gp[3];
+          real r[P];
+          apply<P>(op.hatD, q, r);
+#pragma unroll
+          for (int i = 0; i < P; ++i) { ox[i] = r[i] * jx; oy[i] = r[i] * jy; }
+        } else {
+          const real* gp = &in.vg[le * GS + (xi ? m * P * 5 : m * 5 + 1)];
+          const int gst = xi ? 5 : 5 * P;
+          real qx[P], qy[P];
+#pragma unroll
+          for (int l = 0; l < P; ++l) { qx[l] = q[l] * gp[l * gst]; qy[l] = q[l] * gp[l * gst + 2]; }
+          apply<P>(op.hatD, qx, ox);
+          apply<P>(op.hatD, qy, oy);
+        }
+        real* dx = xi ? s.Fc : s.X;
+        real* dy = xi ? s.Gc : s.Y;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          dx[o + i * st] = f0[0] * op.lbw0[i] + f1[0] * op.lbw1[i] - ox[i];
+          dy[o + i * st] = f0[4 * FS] * op.lbw0[i] + f1[4 * FS] * op.lbw1[i] - oy[i];
+        }
+      }
+      __syncthreads();
+      for (int m = tid; m < n_act * NP; m += T) {
+        const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
+        const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
+        real* gq = a.dQ + size_t(e0 + le) * 8 * NP + node;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const real gx = (s.Fc[k * VS + o] + s.X[k * VS + o]) * iJ, gy = (s.Gc[k * VS + o] + s.Y[k * VS + o]) * iJ;
+          gq[k * NP] = gx;   // the lifted gradient is not local: stored for the stage kernel
+          gq[(4 + k) * NP] = gy;
+          s.Fc[k * VS + o] = gx;
+          s.Gc[k * VS + o] = gy;
+        }
+      }
+      if (a.viscous) {   // gradient traces only feed viscous face fluxes
+        __syncthreads();
+        tile_traces<P, 8, false, Tl>(s.Fc, op.lb0, op.lb1, a.GT + size_t(e0) * FT * 8, n_act, tid);
+        tile_traces<P, 8, false, Tl>(s.Gc, op.lb0, op.lb1, a.GT + size_t(e0) * FT * 8 + 4, n_act, tid);
       }
     }
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    real f = fi[k] - mu_v * fv[k], g = gi[k] - mu_v * gv[k];
-    if (AV && a.av == 1) { f = f - mu_e * ax[k]; g = g - mu_e * ay[k]; }
-    s.Fc[k][le][n] = f * Ja00 + g * Ja10;
-    s.Gc[k][le][n] = f * Ja01 + g * Ja11;
+    if (sense) {
+      __syncthreads();
+      group_sensor<P, EPB, T, real>(a.sensor, ph, op.Vinv, s.Q, s.Fc, VS, s.sens, s_w, n_act, tid, nullptr, flat_g,
+                                    [&](int le, double, double, bool, double g) {
+                                      a.mu_av[e0 + le] = a.av_el[2 * size_t(e0 + le)] * g;
+                                    });
+    }
+    b ^= 1;
+    slot = next_slot;
   }
 }
 
-// Face node t (= side * P + kk) of element le: the side's flux F* dS (signed for a RIGHT side) into
-// s.face[0..3] and, with SIPG / NIPG, the contravariant gradient-face terms into s.face[4..11]
+// Volume flux of a node: F = Fi - (mu + mu_a) Fv (- mu_a grad Q for the Laplacian dissipation, with the
+// element-local gradient), contravariant, into Fc and Gc at o.  gx, gy: gradient of the viscous flux;
+// ax, ay: that of the dissipation.
+template <int VS, bool AV, bool VISC, typename real>
+__device__ __forceinline__ void ns_volume_flux(const Phys<real>& ph, const real* q, const real* gx, const real* gy,
+                                               const real* ax, const real* ay, real mu_v, real mu_l, const real* gp,
+                                               real* Fc, real* Gc) {
+  real fi[4], gi[4], fv[4], gv[4];
+  inviscid_flux(ph, q, fi, gi);
+  if (VISC) viscous_flux(ph, q, gx, gy, fv, gv);
+  const real Ja00 = gp[0], Ja01 = gp[1], Ja10 = gp[2], Ja11 = gp[3];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    real f = fi[k], g = gi[k];
+    if (VISC) { f -= mu_v * fv[k]; g -= mu_v * gv[k]; }
+    if (AV) { f -= mu_l * ax[k]; g -= mu_l * ay[k]; }
+    Fc[k * VS] = f * Ja00 + g * Ja10;
+    Gc[k * VS] = f * Ja01 + g * Ja11;
+  }
+}
+
+// Face task x (element le, side node t): the side's flux F* dS (signed for a RIGHT side) into the side
+// tile and, with SIPG / NIPG, the contravariant gradient-face terms behind it (xi components first)
 // (ComputeRiemannSolver_* and the viscous face loops, DGSpatialDiscretizationMethods.f90:545-1511;
 // DGViscous_BR1.f90:311-371, DGViscous_IP.f90:120-134, 240-247; DGArtificialDissipation.f90:208-249).
-template <int P, int EPB, typename real, bool AFFINE, bool IP, bool AV>
-__device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, NSTiles<P, EPB, real, AFFINE>& s,
-                                             const Phys<real>& ph, int le, int e, int t, real mu_e, bool visc,
-                                             const real* geoE, const real (*own)[EPB][4 * P], bool own_g) {
-  constexpr int NP = P * P;
-  const real mu = ph.mu;
-  const real* lb0 = s.mat + NP;
-  const real* lb1 = lb0 + P;
-  const int sd_ = t / P, kk = t % P;
-  const int4 sd = a.side[size_t(e) * 4 + sd_];
+template <int P, typename Tl, typename real, bool AFFINE, bool IP, bool AV, bool VISC>
+__device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<real>& ph, Tl& s, const typename Tl::In& in,
+                                             const int4* side, int x, int e0) {
+  constexpr int FT = Tl::FT, GS = Tl::GS, FS = Tl::FS, RT = Tl::RT, RG = Tl::RG;
+  const typename Tl::Once& one = s.one;
+  const int le = x / FT, t = x % FT, sd_ = t / P, kk = t % P;
+  real* Fo = &s.F[(le * 4 + sd_) * Tl::PO + kk];
+  const int4 sd = side[le * 4 + sd_];
   const int kind = sd.y & 15;
+  const bool gf = IP && VISC && a.grad_faces;
+  const size_t slot = size_t(e0) * FT + x;
+  real fm[4];   // Ja / J at the side node: contravariant components of the gradient-face terms
+  if (gf) {
+    if (AFFINE) {
+      const real* gp = &in.vg[le * GS];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) fm[k] = gp[k] * gp[4];
+    } else {
+      ld4(a.face_metric + slot * 4, fm);
+    }
+  }
+  const auto grad_terms = [&](const real* Gx, const real* Gy) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const real gx = Gx[k], gy = Gy[k];
+      Fo[(4 + k) * FS] = gx * fm[0] + gy * fm[2];
+      Fo[(8 + k) * FS] = gx * fm[1] + gy * fm[3];
+    }
+  };
   if (kind == SIDE_FLUX) {   // inviscid and viscous flux of the mortar kernel, and its gradient-face terms
-    real fp[4];
-    ld4(a.NF + (size_t(sd.x) * P + kk) * 4, fp);
+    real f[4];
+    ld4(&one.Tn[x * RT], f);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) s.face[k][le][t] = fp[k];
-    if (IP && a.grad_faces && visc) {
-      const real* gp = a.NFG + (size_t(sd.x) * P + kk) * 8;
-      const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-      real fJa00, fJa01, fJa10, fJa11, fiJ;   // metrics and 1/J at the face node
-      if constexpr (AFFINE) { fJa00 = geoE[0]; fJa01 = geoE[1]; fJa10 = geoE[2]; fJa11 = geoE[3]; fiJ = geoE[4]; }
-      else {
-        fJa00 = trace_of(s, s.Ja, 0, le, sd_, kk, lbv);
-        fJa01 = trace_of(s, s.Ja, 1, le, sd_, kk, lbv);
-        fJa10 = trace_of(s, s.Ja, 2, le, sd_, kk, lbv);
-        fJa11 = trace_of(s, s.Ja, 3, le, sd_, kk, lbv);
-        fiJ = real(1) / trace_of(s, s.Ja, 4, le, sd_, kk, lbv);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        s.face[4 + k][le][t] = (gp[k] * fJa00 + gp[4 + k] * fJa10) * fiJ;
-        s.face[8 + k][le][t] = (gp[k] * fJa01 + gp[4 + k] * fJa11) * fiJ;
-      }
+    for (int k = 0; k < 4; ++k) Fo[k * FS] = f[k];
+    if (gf) {
+      real gx[4], gy[4];
+      ld4(&one.GTn[x * RG], gx);
+      ld4(&one.GTn[x * RG + 4], gy);
+      grad_terms(gx, gy);
     }
     return;
   }
-  const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-  real qo[4], gox[4] = {real(0), real(0), real(0), real(0)}, goy[4] = {real(0), real(0), real(0), real(0)};
-  // this element's own traces of the current state (Q, and the gradient when viscous): what the previous
-  // stage (or the prologue, or this stage's gradient kernel) wrote for the neighbours, prefetched
-  cp_async_wait_all();
-#pragma unroll
-  for (int k = 0; k < 4; ++k) qo[k] = own[k][le][t];
-  if (visc) {
-    if (own_g) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { gox[k] = own[4 + k][le][t]; goy[k] = own[8 + k][le][t]; }
-    } else {   // no shared memory left for them: formed here
-      trace4<P, EPB, real>(s.dQ[0], le, sd_, kk, lbv, gox);
-      trace4<P, EPB, real>(s.dQ[1], le, sd_, kk, lbv, goy);
-    }
+  real qo[4], gox[4], goy[4];
+  ld4(&one.To[x * RT], qo);
+  if (VISC) {
+    ld4(&one.GTo[x * RG], gox);
+    ld4(&one.GTo[x * RG + 4], goy);
   }
-  const real* g3 = AFFINE ? a.side_geo + (size_t(e) * 4 + sd_) * 3 : a.side_geo + ((size_t(e) * 4 + sd_) * P + kk) * 3;
-  const real nx = real(g3[0]), ny = real(g3[1]), dS = real(g3[2]);
-  const real invh = real(a.side_invh[size_t(e) * 4 + sd_]);
+  const real* g3 = AFFINE ? &in.vg[le * GS + 8 + sd_ * 3] : &one.sg[x * 3];
+  const real nx = g3[0], ny = g3[1], dS = g3[2], mu = ph.mu;
   // edge viscosity (JumpsBasedEdgeViscosity): mean over the edge's elements; boundary and
-  // periodic edges have one element
-  real mu_ed = mu_e;
-  if (AV && (kind == SIDE_LEFT || kind == SIDE_RIGHT) && sd.z < 0)
-    mu_ed = (real(a.mu_av[sd.x >> 2]) + mu_e) / real(2);
+  // periodic edges have one element (the neighbour's slot then holds this element's)
+  real mu_ed = real(0);
+  if (AV) mu_ed = (real(one.mun[le * 4 + sd_]) + real(in.mu[le])) / real(2);
   const real mu_f = (AV && a.av == 2) ? mu + mu_ed : mu;
-  const real lap = (AV && a.av == 1) ? mu_ed * real(a.side_area[size_t(e) * 4 + sd_]) : real(0);
-  const real penalty = IP ? real(a.sigma0) * mu_f * real(P - 1) * real(P - 1) * invh : real(0);
-  real F[4], Gx[4] = {real(0), real(0), real(0), real(0)}, Gy[4] = {real(0), real(0), real(0), real(0)};
+  const real lap = (AV && a.av == 1) ? mu_ed * real(one.area[le * 4 + sd_]) : real(0);
+  real penalty = real(0);
+  if (IP && VISC) penalty = real(a.sigma0) * mu_f * real(P - 1) * real(P - 1) * real(one.invh[le * 4 + sd_]);
+  real F[4];
   if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
-    real qn[4], gnx[4] = {real(0), real(0), real(0), real(0)}, gny[4] = {real(0), real(0), real(0), real(0)};
-    // the neighbour's traces, prefetched into this task's own face slots (prefetch_neighbour_traces)
-    cp_async_wait_all();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) qn[k] = s.face[k][le][t];
-    if (visc) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { gnx[k] = s.face[4 + k][le][t]; gny[k] = s.face[8 + k][le][t]; }
-    }
     const bool right = kind == SIDE_RIGHT;
-    const real* QL = right ? qn : qo;
-    const real* QR = right ? qo : qn;
+    real qn[4], QL[4], QR[4];
+    ld4(&one.Tn[x * RT], qn);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { QL[k] = right ? qn[k] : qo[k]; QR[k] = right ? qo[k] : qn[k]; }
     int solver = a.riemann;
     if (sd.z >= 0) { const int zr = a.zones[sd.z].riemann; if (zr >= 0) solver = zr; }
-    real Fi[4], FLx[4] = {real(0), real(0), real(0), real(0)}, FLy[4] = {real(0), real(0), real(0), real(0)};
-    real FRx[4] = {real(0), real(0), real(0), real(0)}, FRy[4] = {real(0), real(0), real(0), real(0)};
-    face_riemann(solver, ph, QL, QR, nx, ny, a.FX, (size_t(e) * 4 + sd_) * P + kk, Fi);
-    if (visc) {
-      viscous_flux(ph, QL, right ? gnx : gox, right ? gny : goy, FLx, FLy);
-      viscous_flux(ph, QR, right ? gox : gnx, right ? goy : gny, FRx, FRy);
+    face_riemann(solver, ph, QL, QR, nx, ny, a.FX, slot, F);
+    const real sg = right ? -dS : dS;
+    if (VISC) {
+      real gnx[4], gny[4], ox[4], oy[4], bx[4], by[4];
+      ld4(&one.GTn[x * RG], gnx);
+      ld4(&one.GTn[x * RG + 4], gny);
+      viscous_flux(ph, qo, gox, goy, ox, oy);
+      viscous_flux(ph, qn, gnx, gny, bx, by);
+      const real hm = real(0.5) * mu_f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) F[k] -= hm * (ox[k] + bx[k]) * nx + hm * (oy[k] + by[k]) * ny;
+      if (gf) {
+        real fgx[4], fgy[4], Ax[4], Ay[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { const real d = QL[k] - QR[k]; fgx[k] = d * nx; fgy[k] = d * ny; }
+        viscous_flux(ph, qo, fgx, fgy, Ax, Ay);
+        const real cf = real(0.5) * real(a.epsilon) * mu_f * sg;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { Ax[k] *= cf; Ay[k] *= cf; }
+        grad_terms(Ax, Ay);
+      }
     }
+    const real jump = AV ? penalty + lap : penalty;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      real fv = real(0.5) * (mu_f * FLx[k] + mu_f * FRx[k]) * nx + real(0.5) * (mu_f * FLy[k] + mu_f * FRy[k]) * ny;
-      if (IP) fv = fv - penalty * (QL[k] - QR[k]);
-      if (AV) {
-        const real fa = -(lap * (QL[k] - QR[k]));
-        F[k] = (Fi[k] - fv - fa) * dS;
-      } else {
-        F[k] = (Fi[k] - fv) * dS;
-      }
-      if (right) F[k] = -F[k];
-    }
-    if (IP && a.grad_faces && visc) {
-      real fgx[4], fgy[4], Ax[4], Ay[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { fgx[k] = (QL[k] - QR[k]) * nx; fgy[k] = (QL[k] - QR[k]) * ny; }
-      viscous_flux(ph, right ? QR : QL, fgx, fgy, Ax, Ay);
-      const real cf = (right ? real(-0.5) : real(0.5)) * real(a.epsilon) * mu_f;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { Gx[k] = cf * Ax[k] * dS; Gy[k] = cf * Ay[k] * dS; }
+      if ((IP && VISC) || AV) F[k] += jump * (QL[k] - QR[k]);
+      F[k] *= sg;
     }
   } else {
     const Zone& z = a.zones[sd.z];
     real uB[4], uSB[4];
     const int vbc = bc_states(ph, z, qo, nx, ny, uB, uSB, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
-    real Fi[4];
     if (kind == SIDE_WALL) {
-      euler_wall_flux(ph, qo, nx, ny, dS, Fi);
+      euler_wall_flux(ph, qo, nx, ny, dS, F);
     } else {
       const int solver = z.riemann >= 0 ? z.riemann : a.riemann;
-      face_riemann(solver, ph, qo, uB, nx, ny, a.FX, (size_t(e) * 4 + sd_) * P + kk, Fi);
+      face_riemann(solver, ph, qo, uB, nx, ny, a.FX, slot, F);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) Fi[k] = Fi[k] * dS;
+      for (int k = 0; k < 4; ++k) F[k] = F[k] * dS;
     }
-    real fv[4] = {real(0), real(0), real(0), real(0)};
-    if (vbc != VBC_NEUMANN && visc) {
-      real Fx[4], Fy[4];
-      if (vbc == VBC_ADIABATIC) viscous_flux_adiabatic(ph, qo, qo, gox, goy, Fx, Fy);
-      else viscous_flux(ph, qo, gox, goy, Fx, Fy);
+    if (VISC) {
+      real Gx[4] = {real(0), real(0), real(0), real(0)}, Gy[4] = {real(0), real(0), real(0), real(0)};
+      if (vbc != VBC_NEUMANN) {
+        real Fx[4], Fy[4];
+        if (vbc == VBC_ADIABATIC) viscous_flux_adiabatic(ph, qo, qo, gox, goy, Fx, Fy);
+        else viscous_flux(ph, qo, gox, goy, Fx, Fy);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        fv[k] = (mu_f * Fx[k]) * nx + (mu_f * Fy[k]) * ny;
-        if (IP) fv[k] = fv[k] - penalty * (qo[k] - uSB[k]);
-        fv[k] = fv[k] * dS;
-      }
-      if (IP && a.grad_faces) {
-        real fgx[4], fgy[4], Ax[4], Ay[4];
+        for (int k = 0; k < 4; ++k) {
+          real fv = (mu_f * Fx[k]) * nx + (mu_f * Fy[k]) * ny;
+          if (IP) fv = fv - penalty * (qo[k] - uSB[k]);
+          F[k] -= fv * dS;
+        }
+        if (gf) {
+          real fgx[4], fgy[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { fgx[k] = (qo[k] - uSB[k]) * nx; fgy[k] = (qo[k] - uSB[k]) * ny; }
-        if (vbc == VBC_ADIABATIC) viscous_flux_adiabatic(ph, qo, qo, fgx, fgy, Ax, Ay);
-        else viscous_flux(ph, qo, fgx, fgy, Ax, Ay);
-        const real cf = real(a.epsilon) * mu_f;
+          for (int k = 0; k < 4; ++k) { fgx[k] = (qo[k] - uSB[k]) * nx; fgy[k] = (qo[k] - uSB[k]) * ny; }
+          if (vbc == VBC_ADIABATIC) viscous_flux_adiabatic(ph, qo, qo, fgx, fgy, Gx, Gy);
+          else viscous_flux(ph, qo, fgx, fgy, Gx, Gy);
+          const real cf = real(a.epsilon) * mu_f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { Gx[k] = (cf * Ax[k]) * dS; Gy[k] = (cf * Ay[k]) * dS; }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) F[k] = AV ? Fi[k] - fv[k] - (-(lap * (qo[k] - uSB[k]))) * dS : Fi[k] - fv[k];
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) s.face[k][le][t] = F[k];
-  if (IP && a.grad_faces && visc) {
-    // metrics at the face node (interpolated along the other direction) and contravariant G
-    real fJa00, fJa01, fJa10, fJa11, fiJ;   // metrics and 1/J at the face node (one division, or none)
-    if constexpr (AFFINE) { fJa00 = geoE[0]; fJa01 = geoE[1]; fJa10 = geoE[2]; fJa11 = geoE[3]; fiJ = geoE[4]; }
-    else {
-      fJa00 = trace_of(s, s.Ja, 0, le, sd_, kk, lbv);
-      fJa01 = trace_of(s, s.Ja, 1, le, sd_, kk, lbv);
-      fJa10 = trace_of(s, s.Ja, 2, le, sd_, kk, lbv);
-      fJa11 = trace_of(s, s.Ja, 3, le, sd_, kk, lbv);
-      fiJ = real(1) / trace_of(s, s.Ja, 4, le, sd_, kk, lbv);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      s.face[4 + k][le][t] = (Gx[k] * fJa00 + Gy[k] * fJa10) * fiJ;
-      s.face[8 + k][le][t] = (Gx[k] * fJa01 + Gy[k] * fJa11) * fiJ;
-    }
-  }
-}
-
-// The traces that the face tasks of this thread read (Q traces, and the gradient traces when viscous),
-// copied asynchronously at the start of the launch: the neighbour's into the task's own face slots
-// (face[0..3][le][t] and face[4..11][le][t] belong to face task t alone, which reads them before it
-// writes its fluxes there), this element's own into s.own (the trace buffers hold them: the previous
-// stage's output, the prologue's, or this stage's gradient kernel's), so the copies need no barrier
-// and their latency overlaps the volume phase.  The thread-to-task map is that of the face phase
-// (t = tid, tid + NP, ...).
-template <int P, int EPB, typename real, bool AFFINE>
-__device__ __forceinline__ void prefetch_neighbour_traces(const NSArgs<real>& a, NSTiles<P, EPB, real, AFFINE>& s,
-                                                          real (*own)[EPB][4 * P], bool own_g, int le, int e,
-                                                          int tid, bool active, bool visc) {
-  constexpr int NP = P * P, FT = 4 * P;
-  if (active)
-    for (int t = tid; t < FT; t += NP) {
-      const int sd_ = t / P, kk = t % P;
-      const int4 sd = a.side[size_t(e) * 4 + sd_];
-      const int kind = sd.y & 15;
-      if (kind != SIDE_FLUX) {
-        const size_t slot = (size_t(e) * 4 + sd_) * P + kk;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) cp_async_real(&own[k][le][t], a.T_in + slot * 4 + k);
-        if (visc && own_g) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) cp_async_real(&own[4 + k][le][t], a.GT + slot * 8 + k);
+          for (int k = 0; k < 4; ++k) { Gx[k] = (cf * Gx[k]) * dS; Gy[k] = (cf * Gy[k]) * dS; }
         }
       }
-      if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
-        const int kn = (sd.y & SIDE_REVERSED) ? (P - 1 - kk) : kk;
-        const real* qp = a.T_in + (size_t(sd.x) * P + kn) * 4;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) cp_async_real(&s.face[k][le][t], qp + k);
-        if (visc) {
-          const real* gp = a.GT + (size_t(sd.x) * P + kn) * 8;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) cp_async_real(&s.face[4 + k][le][t], gp + k);
-        }
-      }
+      if (gf) grad_terms(Gx, Gy);
     }
-  cp_async_commit();
+    if (AV)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) F[k] += lap * (qo[k] - uSB[k]) * dS;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) Fo[k * FS] = F[k];
 }
 
-template <int P, int EPB, typename real, bool AFFINE, bool IP, bool AV>
-__global__ void __launch_bounds__(block_of(P, EPB)) ns_stage_kernel(NSArgs<real> a) {
-  constexpr int NP = P * P, FT = 4 * P;
-  constexpr int NW = block_of(P, EPB) / 32;
-  __shared__ NSTiles<P, EPB, real, AFFINE> s;
-  const int flat = threadIdx.x, le = flat / NP, tid = flat - le * NP;
-  const int e = blockIdx.x * EPB + le;
-  const bool active = le < EPB && e < a.n_el;
+// Stage kernel, per group (a barrier between the phases):
+//   A  face nodes and volume nodes as one list of items, faces first in whole warps.  Where the volume flux needs
+//      the element-local gradient (interior penalty with viscous terms; the Laplacian dissipation of a group that
+//      holds an element with viscosity) the nodes only fill the Q tile, else they form their fluxes;
+//   B  (with that gradient) lines: D along both directions; and the gradient-face terms, contracted with hatD along
+//      their side (they enter the lift at every node of a normal line with the same value);
+//   C  (with that gradient) nodes: fluxes;
+//   D  lines: contraction with hatD, lift of the face fluxes (lbw) and the gradient-face terms (lbw, dlbw);
+//   E  nodes: 1/J, RK update, health check;
+//   F  lines: traces of the new state and, on the fused path, of its gradient; then its indicator.
+template <int P, int V, typename real, bool AFFINE, bool IP, bool AV, bool VISC>
+__global__ void __launch_bounds__(ns_threads(P, V), ns_min_ctas<NSTiles<P, V, real, AFFINE, IP, AV, VISC, false>>())
+    ns_stage_kernel(const __grid_constant__ NSArgs<real> a, const __grid_constant__ NSOps<P, real> op) {
+  using Tl = NSTiles<P, V, real, AFFINE, IP, AV, VISC, false>;
+  constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, PO = Tl::PO, VS = Tl::VS, GS = Tl::GS, NF = Tl::NF,
+                FS = Tl::FS;
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  Tl& s = *reinterpret_cast<Tl*>(stage_smem);
+  float* s_w = reinterpret_cast<float*>(stage_smem + sizeof(Tl));
+  const int tid = threadIdx.x, n_groups = (a.n_el + EPB - 1) / EPB;
+  NSPipe<Tl, P, real, AFFINE, IP, AV, VISC, false> pipe{a, s, tid, n_groups};
   Phys<real> ph;
   ph.load(a.pc);
-  const real mu = ph.mu;
-  real geoE[5];
-  const bool visc = a.viscous != 0;
-  // the own traces of the face tasks: Q and gradient where the static shared memory allows (48 KB),
-  // else Q alone (the gradient traces are then formed in the face task)
-  constexpr bool OWN_G = sizeof(s) + size_t(12) * EPB * FT * sizeof(real) <= 48 * 1024;
-  __shared__ real s_own[OWN_G ? 12 : 4][EPB][FT];
-  prefetch_neighbour_traces<P, EPB, real, AFFINE>(a, s, s_own, OWN_G, le, e, tid, active, visc);
-  load_tiles(a, s, flat, le, tid, e, active, geoE);
-  const real mu_e = (AV && active) ? real(a.mu_av[e]) : real(0);
-  // the element gradient feeds the viscous fluxes and the Laplacian dissipation's volume term; an
-  // element without either (mu_e = 0: that term is exactly zero) skips it
-  const bool need_grad = visc || (AV && a.av == 1 && mu_e != real(0));
-  if (IP) {   // the interior-penalty gradient is element-local: recompute it here
-    __syncthreads();
-    element_gradient<P, EPB, real, AFFINE, IP>(a, s, ph, le, tid, e, active && need_grad, geoE);
-  } else if (active) {
-    const real* g = a.dQ + size_t(e) * 8 * NP + tid;
-#pragma unroll
-    for (int d = 0; d < 2; ++d)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) s.dQ[d][k][le][tid] = g[(d * 4 + k) * NP];
-  }
-  __syncthreads();
-  const int i = tid % P, j = tid / P;
-  const real* hatDT = s.mat;   // transposed: hatDT[l * P + i] = hatD(i, l)
-  const real* lb0 = s.mat + NP;
-  const real* lb1 = lb0 + P;
-  const real* lbw0 = lb1 + P;
-  const real* lbw1 = lbw0 + P;
-  const real* dlbw0 = lbw1 + P + NP;
-  const real* dlbw1 = dlbw0 + P;
-  real iJ;
-  if (active) iJ = geoE[4];
-  // Volume fluxes and face fluxes are independent: where an element has at least a quarter of its
-  // threads beyond its 4(N+1) face nodes (N >= 5), those threads form the volume fluxes of all its nodes
-  // while the first 4(N+1) threads form the face fluxes (one barrier fewer, and no thread idles through
-  // the face phase); otherwise each thread forms its own node's volume flux, then the face fluxes.
-  constexpr bool OVERLAP = 4 * (NP - FT) >= NP;
-  if constexpr (OVERLAP) {
-    if (active) {
-      if (tid < FT) ns_face_task<P, EPB, real, AFFINE, IP, AV>(a, s, ph, le, e, tid, mu_e, visc, geoE, s_own, OWN_G);
-      else
-        for (int n = tid - FT; n < NP; n += NP - FT)
-          ns_volume_flux<P, EPB, real, AFFINE, IP, AV>(a, s, ph, le, n, mu_e, need_grad, visc, geoE);
-    }
-  } else {
-    if (active) ns_volume_flux<P, EPB, real, AFFINE, IP, AV>(a, s, ph, le, tid, mu_e, need_grad, visc, geoE);
-    __syncthreads();
-    if (active)
-      for (int t = tid; t < FT; t += NP)
-        ns_face_task<P, EPB, real, AFFINE, IP, AV>(a, s, ph, le, e, t, mu_e, visc, geoE, s_own, OWN_G);
-  }
-  __syncthreads();
-  // The gradient-face terms enter the lift as hatD-contractions along their side, which depend on the
-  // node's index along that side only (Scalar_StdGradientFace): formed once per side node here (P
-  // multiply-adds each) instead of at every node of the element.
-  const bool gf = IP && a.grad_faces && visc;   // uniform over the launch
-  if (gf && active) {
-    for (int t = tid; t < FT; t += NP) {
-      const int sd_ = t / P, kk = t % P;
-      const int row = (sd_ & 1) ? 8 : 4;   // bottom / top: the xi component; right / left: the eta one
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        real d = real(0);
-#pragma unroll
-        for (int l = 0; l < P; ++l) d += hatDT[l * P + kk] * s.face[row + k][le][sd_ * P + l];
-        s.gfd[k][le][t] = d;
-      }
-    }
-  }
-  real qd[4] = {real(0), real(0), real(0), real(0)};
-  if (active) {
-#pragma unroll
-    for (int l = 0; l < P; ++l) {
-      const real hi = hatDT[l * P + i], hj = hatDT[l * P + j];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) qd[k] = qd[k] + hi * s.Fc[k][le][j * P + l] + hj * s.Gc[k][le][l * P + i];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      qd[k] = qd[k] - s.face[k][le][0 * P + i] * lbw0[j];
-      qd[k] = qd[k] - s.face[k][le][1 * P + j] * lbw1[i];
-      qd[k] = qd[k] - s.face[k][le][2 * P + i] * lbw1[j];
-      qd[k] = qd[k] - s.face[k][le][3 * P + j] * lbw0[i];
-    }
-  }
-  if (gf) __syncthreads();
-  if (active) {
-    if (gf) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        qd[k] = qd[k] - (s.gfd[k][le][0 * P + i] * lbw0[j] + s.face[8 + k][le][0 * P + i] * dlbw0[j]);
-        qd[k] = qd[k] - (s.face[4 + k][le][1 * P + j] * dlbw1[i] + s.gfd[k][le][1 * P + j] * lbw1[i]);
-        qd[k] = qd[k] - (s.gfd[k][le][2 * P + i] * lbw1[j] + s.face[8 + k][le][2 * P + i] * dlbw1[j]);
-        qd[k] = qd[k] - (s.face[4 + k][le][3 * P + j] * dlbw0[i] + s.gfd[k][le][3 * P + j] * lbw0[i]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) qd[k] = qd[k] * iJ;
-    const size_t off = (size_t(e) * NP + tid) * 4;
-    if (a.QDot) {
-      double2* dp = reinterpret_cast<double2*>(a.QDot + off);
-      dp[0] = make_double2(double(qd[0]), double(qd[1]));
-      dp[1] = make_double2(double(qd[2]), double(qd[3]));
-    }
-    if (a.update) {
-      real gn[4];
-      if (a.first) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) gn[k] = real(a.b) * qd[k];
+  const bool sense = IP && AV && a.fuse && a.update && a.last && a.sensor.kind != SENSOR_JUMPS;
+  const bool gf = IP && VISC && a.grad_faces, rk = a.update && !a.first;
+  if (sense && a.sensor.kind == SENSOR_LEARNED) sensor_weights_async(s_w, a.sensor.mlp, tid, T);
+  if ((tid & 31) < 4) s.mx[tid & 31][tid >> 5] = 0ull;
+  pipe.start();
+  FlatG flat_g;
+  int b = 0, slot = 0;
+  for (int g = blockIdx.x; g < n_groups; g += gridDim.x) {
+    const int e0 = g * EPB, n_act = pipe.count(g), next_slot = slot == 2 ? 0 : slot + 1;
+    pipe.next(g, rk);
+    typename Tl::In& in = s.in[b];
+    const int4* side = s.side[slot];
+    bool local = IP && VISC;   // the volume fluxes need the element-local gradient (uniform over the CTA)
+    if (AV && !local && a.av == 1)
+      for (int le = 0; le < n_act; ++le) local = local || in.mu[le] != 0.0;
+
+    // A
+    constexpr int NFR = (NF + 31) / 32 * 32;
+    for (int x = tid; x < NFR + Tl::NN; x += T) {
+      if (x < NFR) {
+        if (x < n_act * FT) ns_face_task<P, Tl, real, AFFINE, IP, AV, VISC>(a, ph, s, in, side, x, e0);
       } else {
-        real go[4];
-        ld4(a.G + off, go);
+        const int m = x - NFR, le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
+        if (le >= n_act) continue;
+        double qd[4];
+        ld4(&s.state(b)[m * 4], qd);
+        const real q[4] = {real(qd[0]), real(qd[1]), real(qd[2]), real(qd[3])};
+        if (local || !Tl::KEEP_Q)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) gn[k] = real(a.a) * go[k] + real(a.b) * qd[k];
+          for (int k = 0; k < 4; ++k) s.Q[k * VS + o] = q[k];
+        if (!local) {
+          const real* gp = AFFINE ? &in.vg[le * GS] : &in.vg[le * GS + node * 5];
+          real gx[4], gy[4];
+          if constexpr (VISC && !IP) {
+            const real* gq = &s.one.dQ[le * 8 * NP + node];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { gx[k] = gq[k * NP]; gy[k] = gq[(4 + k) * NP]; }
+          }
+          const real mu_v = (AV && a.av == 2) ? ph.mu + real(in.mu[le]) : ph.mu;
+          if constexpr (!(IP && VISC))
+            ns_volume_flux<VS, false, VISC>(ph, q, gx, gy, gx, gy, mu_v, real(0), gp, &s.Fc[o], &s.Gc[o]);
+        }
       }
-      st4(a.G + off, gn);
-      double2* qp = reinterpret_cast<double2*>(a.Q + off);
-      double2 q01 = qp[0], q23 = qp[1];
-      q01.x = q01.x + a.c * double(gn[0]);
-      q01.y = q01.y + a.c * double(gn[1]);
-      q23.x = q23.x + a.c * double(gn[2]);
-      q23.y = q23.y + a.c * double(gn[3]);
-      qp[0] = q01; qp[1] = q23;
-      check_state(a.health, a.health_host, q01.x, q01.y, q23.x, q23.y, e);
-      s.Q[0][le][tid] = real(q01.x); s.Q[1][le][tid] = real(q01.y);
-      s.Q[2][le][tid] = real(q23.x); s.Q[3][le][tid] = real(q23.y);
     }
+    __syncthreads();
+    pipe.prefetch_rows(g, b, next_slot);
+
+    if (local) {
+      // B
+      tile_derivatives<P>(s, op.D, n_act, tid);
+      if (gf)
+        for (int x = tid; x < n_act * 16; x += T) {   // x = (element, side, variable)
+          const int v = x & 3, sd = (x >> 2) & 3, le = x >> 4;
+          // bottom / top: the xi component along the side; right / left: the eta one
+          real* u = &s.F[(4 + (sd & 1) * 4 + v) * FS + (le * 4 + sd) * PO];
+          real c[P], d[P];
+          load_line<P>(u, 1, c);
+          apply<P>(op.hatD, c, d);
+          store_line<P>(u, 1, d);
+        }
+      __syncthreads();
+      // C
+      for (int m = tid; m < n_act * NP; m += T) {
+        const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
+        const real* gp = AFFINE ? &in.vg[le * GS] : &in.vg[le * GS + node * 5];
+        real q[4], ax[4], ay[4], gx[4], gy[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = s.Q[k * VS + o];
+        node_gradient<P, Tl, AFFINE>(s, gp, o, ax, ay);
+        if constexpr (VISC && !IP) {
+          const real* gq = &s.one.dQ[le * 8 * NP + node];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) { gx[k] = gq[k * NP]; gy[k] = gq[(4 + k) * NP]; }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) { gx[k] = ax[k]; gy[k] = ay[k]; }
+        }
+        const real mu_e = AV ? real(in.mu[le]) : real(0);
+        ns_volume_flux<VS, AV, VISC>(ph, q, gx, gy, ax, ay, (AV && a.av == 2) ? ph.mu + mu_e : ph.mu,
+                                     a.av == 1 ? mu_e : real(0), gp, &s.Fc[o], &s.Gc[o]);
+      }
+      __syncthreads();
+    }
+
+    pipe.prefetch(g, b, next_slot);
+
+    // D
+    for (int x = tid; x < 2 * NF; x += T) {   // x = (direction, variable, element, line)
+      const int y = x % NF, v = y / (P * EPB), le = (y / P) % EPB, m = y % P;
+      if (le >= n_act) continue;
+      const bool xi = x < NF;
+      // the line's end nodes
+      const real* f0 = &s.F[v * FS + (le * 4 + (xi ? 3 : 0)) * PO + m];
+      const real* f1 = &s.F[v * FS + (le * 4 + (xi ? 1 : 2)) * PO + m];
+      real c0 = *f0, c1 = *f1, d0 = real(0), d1 = real(0);
+      if (gf) {   // contracted terms add to the lbw part, the normal components to the dlbw part
+        const int ct = (xi ? 8 : 4) * FS, nt = (xi ? 4 : 8) * FS;
+        c0 += f0[ct];
+        c1 += f1[ct];
+        d0 = f0[nt];
+        d1 = f1[nt];
+      }
+      const auto line = [&](real* u, const int st) {
+        real f[P], r[P];
+        load_line<P>(u, st, f);
+        apply<P>(op.hatD, f, r);
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          r[i] -= c0 * op.lbw0[i];
+          r[i] -= c1 * op.lbw1[i];
+          if (IP && VISC) {
+            r[i] -= d0 * op.dlbw0[i];
+            r[i] -= d1 * op.dlbw1[i];
+          }
+        }
+        store_line<P>(u, st, r);
+      };
+      if (xi) line(&s.Fc[v * VS + (le * P + m) * PO], 1);
+      else line(&s.Gc[v * VS + le * P * PO + m], PO);
+    }
+    __syncthreads();
+
+    // E
+    if (rk) pipe.wait(1);
+    for (int m = tid; m < (Tl::NN + 31) / 32 * 32; m += T) {
+      const bool on = m < n_act * NP;
+      const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
+      const size_t off = (size_t(e0) * NP + m) * 4;
+      real qd[4] = {real(0), real(0), real(0), real(0)};
+      if (on) {
+        const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) qd[k] = (s.Fc[k * VS + o] + s.Gc[k * VS + o]) * iJ;
+      }
+      if (a.resid)   // the whole warp takes part
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned long long w = warp_max_bits(fabs(double(qd[k])));
+          if ((tid & 31) == 0 && w > s.mx[k][tid >> 5]) s.mx[k][tid >> 5] = w;
+        }
+      if (!on) continue;
+      if (a.QDot) {
+        const double dq[4] = {double(qd[0]), double(qd[1]), double(qd[2]), double(qd[3])};
+        st4(a.QDot + off, dq);
+      }
+      if (a.update) {
+        real gn[4];
+        if (a.first) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gn[k] = real(a.b) * qd[k];
+        } else {
+          ld4(&s.G[m * 4], gn);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gn[k] = real(a.a) * gn[k] + real(a.b) * qd[k];
+        }
+        st4(a.G + off, gn);
+        double q[4];
+        if constexpr (Tl::KEEP_Q) {
+          ld4(&in.Q[m * 4], q);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) q[k] = double(s.Q[k * VS + o]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = q[k] + a.c * double(gn[k]);
+        st4(a.Q + off, q);
+        check_state(a.health, a.health_host, q[0], q[1], q[2], q[3], e0 + le);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s.Q[k * VS + o] = real(q[k]);
+      }
+    }
+
+    // F
+    if (a.update) {
+      __syncthreads();
+      real* T_out = a.T_out + size_t(e0) * FT * 4;
+      if (IP && VISC && a.fuse)   // the side tile is free since the lift
+        gradient_traces<P, AFFINE>(s, op, in.vg, T_out, a.GT_out + size_t(e0) * FT * 8, n_act, tid);
+      else
+        tile_traces<P, 4, !IP, Tl>(s.Q, op.lb0, op.lb1, T_out, n_act, tid);
+      if constexpr (IP && AV) {
+        if (sense) {
+          __syncthreads();
+          group_sensor<P, EPB, T, real>(a.sensor, ph, op.Vinv, s.Q, s.Fc, VS, s.sens, s_w, n_act, tid, nullptr, flat_g,
+                                        [&](int le, double, double, bool, double g) {
+                                          a.mu_next[e0 + le] = a.av_el[2 * size_t(e0 + le)] * g;
+                                        });
+        }
+      }
+    }
+    b ^= 1;
+    slot = next_slot;
   }
   if (a.resid) {
-    double m[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) m[k] = active ? fabs(double(qd[k])) : 0.0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) m[k] = nanmax(m[k], __shfl_xor_sync(0xffffffffu, m[k], off));
-    if ((flat & 31) == 0)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) s.red[flat >> 5][k] = m[k];
-  }
-  __syncthreads();
-  if (a.resid && flat < 4) {
-    double mx = 0.0;
-    for (int w = 0; w < NW; ++w) mx = nanmax(mx, s.red[w][flat]);
-    a.resid[size_t(blockIdx.x) * 4 + flat] = mx;
-  }
-  if (active && a.update) {
-    for (int t = tid; t < FT; t += NP) {
-      const int sd_ = t / P, kk = t % P;
-      const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-      real tr[4];
-      trace4<P, EPB, real>(s.Q, le, sd_, kk, lbv, tr);
-      st4(a.T_out + ((size_t(e) * 4 + sd_) * P + kk) * 4, tr);
-      if (IP && AFFINE && a.fuse && visc) {   // the face tiles are dead since the lift
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s.face[k][le][t] = tr[k];
-      }
-    }
-  }
-  if (IP && AFFINE && a.fuse && a.update && visc && flat < 2 * P) {
-    const int sdt = flat / P, l = flat % P;
-    const real* lbv = sdt == 0 ? lb0 : lb1;
-    const real* DT = lbw1 + P;   // transposed D: DT[l * P + i] = D(i, l)
-    real d = real(0);
-#pragma unroll
-    for (int m = 0; m < P; ++m) d += lbv[m] * DT[l * P + m];
-    s.dl[sdt][l] = d;
-  }
-  if constexpr (IP) {
-    // Fused interior penalty: what the next stage's neighbours read of this element's new state --
-    // its gradient traces (the local gradient, ComputeInteriorGradient, interpolated to the sides) and,
-    // after the last stage of a step, its element-local indicator.  a.fuse, a.update, a.viscous and
-    // a.last are uniform over the launch.
-    if (a.fuse && a.update) {
-      __syncthreads();   // every node's new state is in s.Q (and, affine, its traces in s.face[0..3])
-      if (visc && AFFINE) {
-        // Affine element: the traces of the gradient straight from the new state.  Along the side, the
-        // derivative of the side's Q traces (D applied to them); across it, each normal line of nodes
-        // contracted with lb^T D.  The same as the nodal gradient interpolated to the side, without
-        // forming the gradient at every node.
-        if (active) {
-          const real* DT = lbw1 + P;   // transposed D
-          for (int t = tid; t < FT; t += NP) {
-            const int sd_ = t / P, kk = t % P;
-            const real* dlv = s.dl[(sd_ == 0 || sd_ == 3) ? 0 : 1];
-            real dt_[4] = {real(0), real(0), real(0), real(0)}, dn[4] = {real(0), real(0), real(0), real(0)};
-#pragma unroll
-            for (int l = 0; l < P; ++l) {
-              const real dk = DT[l * P + kk];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) dt_[k] += dk * s.face[k][le][sd_ * P + l];
-            }
-#pragma unroll
-            for (int m = 0; m < P; ++m) {
-              const int l = trace_step<real>(P, m, kk);
-              const int node = face_node(P, sd_, l, kk);
-              const real w = dlv[l];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) dn[k] += w * s.Q[k][le][node];
-            }
-            // bottom / top: along the side is xi; right / left: along the side is eta
-            const bool alongXi = sd_ == 0 || sd_ == 2;
-            const real Ja00 = geoE[0], Ja01 = geoE[1], Ja10 = geoE[2], Ja11 = geoE[3], iJ = geoE[4];
-            real tx[4], ty[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const real dxi = alongXi ? dt_[k] : dn[k], deta = alongXi ? dn[k] : dt_[k];
-              tx[k] = (dxi * Ja00 + deta * Ja01) * iJ;
-              ty[k] = (dxi * Ja10 + deta * Ja11) * iJ;
-            }
-            real* gp = a.GT_out + ((size_t(e) * 4 + sd_) * P + kk) * 8;
-            st4(gp, tx);
-            st4(gp + 4, ty);
-          }
-        }
-      } else if (visc) {
-        element_gradient<P, EPB, real, AFFINE, IP>(a, s, ph, le, tid, e, active, geoE);
-        __syncthreads();
-        if (active) {
-          for (int t = tid; t < FT; t += NP) {
-            const int sd_ = t / P, kk = t % P;
-            const real* lbv = (sd_ == 0 || sd_ == 3) ? lb0 : lb1;
-            real* gp = a.GT_out + ((size_t(e) * 4 + sd_) * P + kk) * 8;
-            real tx[4], ty[4];
-            trace4<P, EPB, real>(s.dQ[0], le, sd_, kk, lbv, tx);
-            trace4<P, EPB, real>(s.dQ[1], le, sd_, kk, lbv, ty);
-            st4(gp, tx);
-            st4(gp + 4, ty);
-          }
-        }
-      }
-      if (AV && a.last && a.sensor.kind != SENSOR_JUMPS) {
-        const int n_active = a.n_el - int(blockIdx.x) * EPB < EPB ? a.n_el - int(blockIdx.x) * EPB : EPB;
-        // the gradient, contravariant-flux and face tiles (contiguous) are dead here: where they are
-        // large enough they hold the indicator's scratch, which keeps the kernel's static shared memory
-        // within 48 KB (FP64 at high and low orders); otherwise the indicator declares its own
-        constexpr size_t dead = sizeof(s.dQ) + sizeof(s.Fc) + sizeof(s.Gc) + sizeof(s.face) + sizeof(s.gfd);
-        constexpr bool lend = dead >= sensor_ext_bytes<P, EPB, real>();
-        __syncthreads();   // the gradient traces above have read s.dQ (affine: s.face)
-        const SensorOut so = element_sensor<P, EPB, real, lend>(a.sensor, ph, s.Q, n_active, s.mat + 2 * NP + 7 * P,
-                                                                le, tid, active, nullptr, &s.dQ[0][0][0][0]);
-        if (active && tid == 0) a.mu_next[e] = a.av_el[2 * size_t(e)] * so.g;
-      }
+    __syncthreads();
+    if (tid < 4) {
+      unsigned long long m = 0ull;
+      for (int w = 0; w < T / 32; ++w) m = s.mx[tid][w] > m ? s.mx[tid][w] : m;
+      a.resid[size_t(blockIdx.x) * 4 + tid] = __longlong_as_double((long long)m);
     }
   }
 }

@@ -67,6 +67,9 @@ struct StageArgs {
   PhysConst pc;
 };
 
+__host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
+__host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
+
 // Metrics record of an element, a multiple of 16 bytes long in either precision.  Curved: [P*P][5] with
 // Ja00 Ja01 Ja10 Ja11 1/J per node.  Affine (AFFINE_REC reals): those five, three unused, then nx ny dS of
 // the four sides.
@@ -161,6 +164,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   return false;
 }
 
+// Max over the warp of non-negative values, as bits (ordered as the values are; NaN above all): two 32-bit
+// reductions.
+__device__ __forceinline__ unsigned long long warp_max_bits(double v) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  const unsigned hi = unsigned(u >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? unsigned(u) : 0u);
+  return (static_cast<unsigned long long>(mh) << 32) | ml;
+}
+
 // max that keeps NaN (a residual that is NaN must stay visible)
 __device__ __forceinline__ double nanmax(double m, double v) { return (v > m || v != v) ? v : m; }
 
@@ -186,15 +198,6 @@ __device__ __forceinline__ void check_state(int* health, int* health_host, doubl
 __host__ __device__ constexpr int face_node(int P, int side, int l, int kk) {
   return (side == 0 || side == 2) ? (l * P + kk) : (kk * P + l);
 }
-// Order of the P terms of a Navier-Stokes trace at face node kk: step m takes line node l = (m + kk) mod P.
-// The face nodes of a side sit in consecutive lanes; without the rotation the lanes of a right or left side
-// (a column of the tile) would read one column at a time, P words apart, into the same banks.
-__host__ __device__ constexpr int trace_l(int P, int m, int kk) { return (m + kk) % P; }
-// The rotation is used in double, where a column side's lanes collide 4 ways; in float they collide 2
-// ways and the rotated (runtime) addressing costs more registers than the conflicts cost time.
-template <typename real>
-__host__ __device__ constexpr int trace_step(int P, int m, int kk) { return sizeof(real) == 8 ? trace_l(P, m, kk) : m; }
-
 // Shared memory of a stage CTA.
 template <int P, int V, typename real, bool AFFINE, bool LGL>
 struct StageTiles {
@@ -485,11 +488,13 @@ __global__ void __launch_bounds__(stage_threads(P, V))
 }
 
 // Traces of the resident state (after hg_set_state).
-// rotated: the summation order of the Navier-Stokes stage kernels (trace_step), else that of the Euler
-// stage kernel, so that a state loaded from the host has the traces bit for bit that a stage left.
+// Summed in the order of the stage kernels, so that a state loaded from the host has the traces bit for bit that
+// a stage left.  how = TRACE_NODAL: the Euler kernel's Gauss-Lobatto traces, the end nodes themselves;
+// TRACE_RELATIVE: BR1's, in float relative to the line's first node.
+enum { TRACE_PLAIN = 0, TRACE_NODAL = 1, TRACE_RELATIVE = 2 };
 template <int P, int EPB, typename real>
 __global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const double* Q, const double* mats, real* T,
-                                                             bool rotated) {
+                                                             int how) {
   constexpr int NP = P * P;
   constexpr int FT = 4 * P;
   __shared__ real s_lb[2 * P];
@@ -508,11 +513,20 @@ __global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const dou
     const int s = t / P, kk = t % P;
     const real* lbv = (s == 0 || s == 3) ? s_lb : s_lb + P;
     real tr[4] = {real(0), real(0), real(0), real(0)};
-    for (int m = 0; m < P; ++m) {
-      const int l = rotated ? trace_step<real>(P, m, kk) : m;
-      const int node = face_node(P, s, l, kk);
+    if (how == TRACE_NODAL) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) tr[k] += s_Q[k][le][node] * lbv[l];
+      for (int k = 0; k < 4; ++k) tr[k] = s_Q[k][le][face_node(P, s, (s == 0 || s == 3) ? 0 : P - 1, kk)];
+    } else if (sizeof(real) == 8 || how == TRACE_PLAIN) {
+      for (int l = 0; l < P; ++l)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tr[k] += s_Q[k][le][face_node(P, s, l, kk)] * lbv[l];
+    } else {
+      const int n0 = face_node(P, s, 0, kk);
+      for (int l = 1; l < P; ++l)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tr[k] += (s_Q[k][le][face_node(P, s, l, kk)] - s_Q[k][le][n0]) * lbv[l];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) tr[k] = s_Q[k][le][n0] + tr[k];
     }
     real* tp = T + ((size_t(e) * 4 + s) * P + kk) * 4;
 #pragma unroll
