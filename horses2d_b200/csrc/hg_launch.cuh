@@ -21,6 +21,23 @@ static int resident_ctas(const hg_ctx* c, std::atomic<int>* known, K kernel, int
   return n;
 }
 
+// Launch that may overlap the end of the kernel before it on the stream (grid_wait, hg_stage.cuh).  Not under
+// per-kernel timing, whose events stand between the kernels.
+template <typename... KA, typename... A>
+static void launch_dependent(hg_ctx* c, void (*kernel)(KA...), int grid, int threads, size_t smem, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = c->prof ? 0 : 1;
+  HG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 template <int P, typename real>
 static StageOps<P, real> stage_ops(const hg_ctx* c) {
   StageOps<P, real> o;
@@ -46,7 +63,7 @@ static void launch_stage_PAL(hg_ctx* c, const StageArgs<real>& a) {
   const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
   if (a.resid) c->n_resid = grid;
   const StageOps<P, real> op = stage_ops<P, real>(c);
-  timed(c, HG_KERNEL_STAGE, [&] { stage_kernel<P, V, real, AFFINE, LGL><<<grid, Tl::T, sizeof(Tl), c->stream>>>(a, op); });
+  timed(c, HG_KERNEL_STAGE, [&] { launch_dependent(c, stage_kernel<P, V, real, AFFINE, LGL>, grid, Tl::T, sizeof(Tl), a, op); });
   ++c->launches;
 }
 
@@ -107,7 +124,7 @@ static int launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind,
   const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
   const int most = c->n_sm * std::min(32, resident_ctas(c, known, kernel, Tl::T, smem));
   const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
-  timed(c, kind, [&] { kernel<<<grid, Tl::T, smem, c->stream>>>(a, op); });
+  timed(c, kind, [&] { launch_dependent(c, kernel, grid, Tl::T, smem, a, op); });
   ++c->launches;
   return grid;
 }
@@ -125,7 +142,7 @@ static void launch_ns_PAI(hg_ctx* c, const NSArgs<real>& a) {
     EdgeWeights<P, real> ew;
     for (int k = 0; k < P; ++k) ew.w[k] = op.w[k];
     const int grid = (a.n_el + jumps_epb(P) - 1) / jumps_epb(P);
-    timed(c, HG_KERNEL_GRADIENT, [&] { jumps_kernel<P, real, AFFINE><<<grid, 128, 0, c->stream>>>(a, ew); });
+    timed(c, HG_KERNEL_GRADIENT, [&] { launch_dependent(c, jumps_kernel<P, real, AFFINE>, grid, 128, 0, a, ew); });
     ++c->launches;
   }
   if (a.run_stage) {

@@ -204,7 +204,8 @@ struct NSPipe {
     if (a.health_host) *reinterpret_cast<volatile int*>(a.health_host) = 1;
   }
   // inputs of group g (those of struct In into half b), and the side table of the group after it (thread 0)
-  __device__ __forceinline__ void bulk(int g, int b, bool own_side, int slot) const {
+  // first: of the CTA's first group, where the constant ones (tables, metrics) go ahead of the wait for the kernel before
+  __device__ __forceinline__ void bulk(int g, int b, bool first, int slot) const {
     constexpr unsigned R = sizeof(real);
     const int e0 = g * EPB, n = count(g), gn = g + gridDim.x;
     typename Tl::In& in = s.in[b];
@@ -212,27 +213,30 @@ struct NSPipe {
     const unsigned bq = n * NP * 32u;
     const unsigned bd = !GRAD && !IP ? n * NP * 8u * R : 0u, bv = n * GS * R, bs = !AFFINE && Tl::FACES ? n * FT * 3u * R : 0u;
     const unsigned bh = IP && VISC && !GRAD ? n * 32u : 0u, ba = AV && !GRAD ? n * 32u : 0u;
-    const unsigned b0 = own_side ? n * 64u : 0u, bn = gn < n_groups ? count(gn) * 64u : 0u;
+    const unsigned b0 = first ? n * 64u : 0u, bn = gn < n_groups ? count(gn) * 64u : 0u;
     mbar_expect(bar, bq + bd + bv + bs + bh + ba + b0 + bn);
-    bulk_copy(const_cast<double*>(s.state(b)), a.Q + size_t(e0) * NP * 4, bq, bar);
     if (b0) bulk_copy(s.side[slot], a.side + size_t(e0) * 4, b0, bar);
-    if (bd) bulk_copy(s.one.dQ, a.dQ + size_t(e0) * NP * 8, bd, bar);
     bulk_copy(in.vg, a.vol_geo + size_t(e0) * GS, bv, bar);
     if (bs) bulk_copy(s.one.sg, a.side_geo + size_t(e0) * FT * 3, bs, bar);
     if (bh) bulk_copy(s.one.invh, a.side_invh + size_t(e0) * 4, bh, bar);
     if (ba) bulk_copy(s.one.area, a.side_area + size_t(e0) * 4, ba, bar);
     if (bn) bulk_copy(s.side[slot == 2 ? 0 : slot + 1], a.side + size_t(gn) * EPB * 4, bn, bar);
+    if (first) grid_wait();
+    bulk_copy(const_cast<double*>(s.state(b)), a.Q + size_t(e0) * NP * 4, bq, bar);
+    if (bd) bulk_copy(s.one.dQ, a.dQ + size_t(e0) * NP * 8, bd, bar);
   }
+  __device__ __forceinline__ int4 side_of(const int4* side, int x) const { return side[(x / FT) * 4 + (x % FT) / P]; }
   // the side-node records of group g, each copied and read by one thread; the viscosities of the group's elements
   // (into half b) and of their neighbours
-  __device__ __forceinline__ void rows(int g, int b, const int4* side) const {
+  // (at0: the side-table entry of the thread's first task)
+  __device__ __forceinline__ void rows(int g, int b, const int4* side, int4 at0) const {
     constexpr int RT = Tl::RT, RG = Tl::RG;
     typename Tl::Once& one = s.one;
     const int n = count(g);
     if (Tl::FACES)
       for (int x = tid; x < n * FT; x += T) {
-        const int t = x % FT, kk = t % P;
-        const int4 sd = side[(x / FT) * 4 + t / P];
+        const int kk = x % P;
+        const int4 sd = x == tid ? at0 : side_of(side, x);
         const int kind = sd.y & 15;
         const size_t own = size_t(g) * EPB * FT + x;
         if (kind != SIDE_FLUX) {
@@ -273,9 +277,12 @@ struct NSPipe {
     if (tid == 0) {
       for (int k = 0; k < 2; ++k) mbar_init(&s.bar[k]);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      bulk(blockIdx.x, 0, true, 0);
     }
-    rows(blockIdx.x, 0, a.side + size_t(blockIdx.x) * EPB * 4);
+    const int4* side0 = a.side + size_t(blockIdx.x) * EPB * 4;
+    const int4 at0 = tid < count(blockIdx.x) * FT ? side_of(side0, tid) : make_int4(0, 0, 0, 0);
+    if (tid == 0) bulk(blockIdx.x, 0, true, 0);
+    else grid_wait();
+    rows(blockIdx.x, 0, side0, at0);
     __syncthreads();   // the barriers are initialised
   }
   __device__ __forceinline__ void wait(int k) {
@@ -288,6 +295,7 @@ struct NSPipe {
     wait(0);
     cp_async_wait_all();
     __syncthreads();
+    if (g + int(gridDim.x) >= n_groups) grid_launch_next();   // the CTA's last group
     if (rk && tid == 0) {
       const unsigned bytes = count(g) * NP * 4u * unsigned(sizeof(real));
       mbar_expect(&s.bar[1], bytes);
@@ -296,7 +304,9 @@ struct NSPipe {
   }
   // after the barrier behind the face tasks: the next group's records
   __device__ __forceinline__ void prefetch_rows(int g, int b, int next_slot) const {
-    if (g + int(gridDim.x) < n_groups) rows(g + gridDim.x, b ^ 1, s.side[next_slot]);
+    const int gn = g + int(gridDim.x);
+    if (gn < n_groups)
+      rows(gn, b ^ 1, s.side[next_slot], tid < count(gn) * FT ? side_of(s.side[next_slot], tid) : make_int4(0, 0, 0, 0));
   }
   // after the barrier behind the last use of struct Once: the rest of the next group's inputs
   __device__ __forceinline__ void prefetch(int g, int b, int next_slot) const {
@@ -442,6 +452,8 @@ __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSAr
   Phys<real> ph;
   ph.load(a.pc);
   __syncthreads();
+  grid_wait();
+  grid_launch_next();
   if (tid < n_act * FT) {
     const int sd_ = (tid % FT) / P, kk = tid % P;
     const size_t sbase = size_t(e0) * 4 + tid / P, slot = size_t(e0) * FT + tid;

@@ -151,6 +151,12 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned b
                    static_cast<unsigned>(__cvta_generic_to_shared(dst))), "l"(src), "r"(bytes),
                "r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))) : "memory");
 }
+// Programmatic dependent launch: a kernel launched behind another one on the stream may start while that one
+// still runs; what it reads or overwrites of the other's data comes after grid_wait.  A stage takes 4 us on a small
+// mesh, a third of it between the last store of one kernel and the first load of the next.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // Waits for the phase; gives up after a bounded number of polls (each suspends the thread for a while) and
 // reports false, so that a copy which never lands ends the launch instead of hanging it.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
@@ -239,30 +245,34 @@ __global__ void __launch_bounds__(stage_threads(P, V))
   ph.load(a.pc);
 
   const auto count = [&](int g) { return min(EPB, a.n_el - g * EPB); };
-  // inputs of group g into half b, and the side table of the group after it (thread 0)
-  const auto issue_bulk = [&](int g, int b, bool own_side, int slot) {
+  // inputs of group g into half b, and the side table of the group after it (thread 0).  first: of the CTA's first
+  // group, where the constant ones (tables, metrics) go ahead of the wait for the kernel before
+  const auto issue_bulk = [&](int g, int b, bool first, int slot) {
     const int e0 = g * EPB, n = count(g), gn = g + gridDim.x;
     const bool rk = a.update && !a.first;
     typename Tl::In& in = s.in[b];
     const unsigned bq = n * NP * 32u, bg = rk ? n * NP * 4u * sizeof(real) : 0u, bt = LGL ? 0u : n * FT * 4u * sizeof(real);
     const unsigned bv = n * GS * unsigned(sizeof(real)), bs = AFFINE ? 0u : n * FT * 3u * sizeof(real);
-    const unsigned b0 = own_side ? n * 64u : 0u, bn = gn < n_groups ? count(gn) * 64u : 0u;
+    const unsigned b0 = first ? n * 64u : 0u, bn = gn < n_groups ? count(gn) * 64u : 0u;
     uint64_t* bar = &s.bar[b];
     mbar_expect(bar, bq + bg + bt + bv + bs + b0 + bn);
-    bulk_copy(in.Q, a.Q + size_t(e0) * NP * 4, bq, bar);
     if (b0) bulk_copy(s.side[slot], a.side + size_t(e0) * 4, b0, bar);
-    if (bt) bulk_copy(in.To, a.T_in + size_t(e0) * FT * 4, bt, bar);
     bulk_copy(in.vg, a.vol_geo + size_t(e0) * GS, bv, bar);
     if (bs) bulk_copy(in.sg, a.side_geo + size_t(e0) * FT * 3, bs, bar);
-    if (bg) bulk_copy(in.G, a.G + size_t(e0) * NP * 4, bg, bar);
     if (bn) bulk_copy(s.side[slot == 2 ? 0 : slot + 1], a.side + size_t(gn) * EPB * 4, bn, bar);
+    if (first) grid_wait();
+    bulk_copy(in.Q, a.Q + size_t(e0) * NP * 4, bq, bar);
+    if (bt) bulk_copy(in.To, a.T_in + size_t(e0) * FT * 4, bt, bar);
+    if (bg) bulk_copy(in.G, a.G + size_t(e0) * NP * 4, bg, bar);
   };
   // the neighbours' traces of group g into half b: a face task's copy is issued and read by one thread
-  const auto issue_rows = [&](int g, int b, const int4* side) {
+  // (at0: the table entry of the thread's first task)
+  const auto side_of = [&](const int4* side, int x) { return side[(x / FT) * 4 + (x % FT) / P]; };
+  const auto issue_rows = [&](int g, int b, const int4* side, int4 at0) {
     const int n = count(g) * FT;
     for (int x = tid; x < n; x += T) {
-      const int t = x % FT, kk = t % P;
-      const int4 sd = side[(x / FT) * 4 + t / P];
+      const int kk = x % P;
+      const int4 sd = x == tid ? at0 : side_of(side, x);
       const int kind = sd.y & 15;
       if (kind == SIDE_LEFT || kind == SIDE_RIGHT)
         cp_async_4(&s.in[b].Tn[x * 4], a.T_in + (size_t(sd.x) * P + ((sd.y & SIDE_REVERSED) ? P - 1 - kk : kk)) * 4);
@@ -276,9 +286,12 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     mbar_init(&s.bar[0]);
     mbar_init(&s.bar[1]);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    issue_bulk(blockIdx.x, 0, true, 0);
   }
-  issue_rows(blockIdx.x, 0, a.side + size_t(blockIdx.x) * EPB * 4);
+  const int4* side0 = a.side + size_t(blockIdx.x) * EPB * 4;
+  const int4 at0 = tid < count(blockIdx.x) * FT ? side_of(side0, tid) : make_int4(0, 0, 0, 0);
+  if (tid == 0) issue_bulk(blockIdx.x, 0, true, 0);
+  else grid_wait();
+  issue_rows(blockIdx.x, 0, side0, at0);
   if (a.resid)
 #pragma unroll
     for (int k = 0; k < 4; ++k) s.mx[k][tid] = 0.0;
@@ -298,7 +311,9 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     const int next_slot = slot == 2 ? 0 : slot + 1;
     if (g + int(gridDim.x) < n_groups) {
       if (tid == 0) issue_bulk(g + gridDim.x, b ^ 1, false, next_slot);
-      issue_rows(g + gridDim.x, b ^ 1, s.side[next_slot]);
+      issue_rows(g + gridDim.x, b ^ 1, s.side[next_slot], tid < count(g + gridDim.x) * FT ? side_of(s.side[next_slot], tid) : at0);
+    } else {
+      grid_launch_next();   // the CTA's last group
     }
     const typename Tl::In& in = s.in[b];
     const int4* side = s.side[slot];
