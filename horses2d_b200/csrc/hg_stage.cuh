@@ -114,6 +114,22 @@ __device__ __forceinline__ void st4(double* p, const double* v) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
+// W = 2 or 4 of them.
+template <typename real, int W>
+__device__ __forceinline__ void ld_w(const real* p, real (&o)[W]) {
+  if constexpr (W == 4) {
+    ld4(p, o);
+  } else {
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    o[0] = v.x; o[1] = v.y;
+  }
+}
+template <typename real, int W>
+__device__ __forceinline__ void st_w(real* p, const real (&v)[W]) {
+  if constexpr (W == 4) st4(p, v);
+  else *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+}
+
 // One value from global into shared memory as an asynchronous copy (4 or 8 bytes); the issuing thread
 // sees it after cp_async_wait_all.
 __device__ __forceinline__ void cp_async_real(float* dst, const float* src) {
@@ -170,6 +186,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   return false;
 }
 
+// max that keeps NaN (a residual that is NaN must stay visible)
+__device__ __forceinline__ double nanmax(double m, double v) { return (v > m || v != v) ? v : m; }
+
+// Per-CTA residual maxima from each lane's W variables (W = 2: even lanes 0 and 1, odd lanes 2 and 3); scratch holds
+// W T values.
+template <int W, int T>
+__device__ __forceinline__ void residual_partial(const double* mx, double* scratch, double* out, int tid) {
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < W; ++k) scratch[W * tid + k] = mx[k];
+  __syncthreads();
+  if (tid < 4) {
+    double m = 0.0;
+    for (int t = tid; t < W * T; t += 4) m = nanmax(m, scratch[t]);
+    out[tid] = m;
+  }
+}
+
 // Max over the warp of non-negative values, as bits (ordered as the values are; NaN above all): two 32-bit
 // reductions.
 __device__ __forceinline__ unsigned long long warp_max_bits(double v) {
@@ -178,9 +212,6 @@ __device__ __forceinline__ unsigned long long warp_max_bits(double v) {
   const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? unsigned(u) : 0u);
   return (static_cast<unsigned long long>(mh) << 32) | ml;
 }
-
-// max that keeps NaN (a residual that is NaN must stay visible)
-__device__ __forceinline__ double nanmax(double m, double v) { return (v > m || v != v) ? v : m; }
 
 // Health of an updated node state.  The reference stops with "The simulation has crashed" when Q holds
 // a NaN (DGTimeIntegrator.f90:224-233); here every RK update checks its node: bit 1 a non-finite value,
@@ -223,7 +254,6 @@ struct StageTiles {
   alignas(16) int4 side[3][EPB * 4];
   real Fc[4 * VS], Gc[4 * VS];      // contravariant fluxes, then their contractions; Fc then holds the new state
   real F[4 * NF];                   // face fluxes x dS (signed for a RIGHT side)
-  double mx[4][T];                  // per-thread max |QDot|
   uint64_t bar[2];
 };
 
@@ -292,9 +322,8 @@ __global__ void __launch_bounds__(stage_threads(P, V))
   if (tid == 0) issue_bulk(blockIdx.x, 0, true, 0);
   else grid_wait();
   issue_rows(blockIdx.x, 0, side0, at0);
-  if (a.resid)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) s.mx[k][tid] = 0.0;
+  constexpr int W = sizeof(real) == 8 ? 2 : 4;   // variables to a lane in phase C
+  double mx[W] = {};                            // max |QDot| of this lane's variables
   __syncthreads();   // the barriers are initialised
 
   int b = 0, slot = 0;
@@ -420,49 +449,66 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     }
     __syncthreads();
 
-    // C: time derivative and update
-    for (int m = tid; m < n_act * NP; m += T) {
-      const int le = m / NP, node = m % NP, i = node % P, j = node / P;
-      const size_t off = (size_t(e0) * NP + m) * 4;
-      const int o = (le * P + j) * PO + i;
-      const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
-      real qd[4];
+    // C: time derivative and update, W variables of a node to a lane.  In double two lanes share a node: 16-byte
+    // records side by side over the lanes, in shared memory as in HBM (16 x 16 elements 12.3 -> 10.8 us a step,
+    // orders 5 and 7 with mortars 4.4 -> 4.2 ms; in float, whose records are half as long, a lane per node is the
+    // faster one: 128 vortex boxes 2.44 against 2.66 ms)
+    for (int x = tid; x < (4 / W * Tl::NN + 31) / 32 * 32; x += T) {
+      const int m = x / (4 / W), h = x % (4 / W) * W;
+      const bool on = m < n_act * NP;
+      const int le = m / NP, node = m % NP, i = node % P, j = node / P, o = (m / P) * PO + node % P;
+      const size_t off = (size_t(e0) * NP + m) * 4 + h;
+      real qd[W] = {};
+      if (on) {
+        const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) qd[k] = (s.Fc[k * VS + o] + s.Gc[k * VS + o]) * iJ;
-      if (a.QDot) {
-        const double dq[4] = {double(qd[0]), double(qd[1]), double(qd[2]), double(qd[3])};
-        st4(a.QDot + off, dq);
+        for (int k = 0; k < W; ++k) qd[k] = (s.Fc[(h + k) * VS + o] + s.Gc[(h + k) * VS + o]) * iJ;
+        if (a.QDot) {
+          double dq[W];
+#pragma unroll
+          for (int k = 0; k < W; ++k) dq[k] = double(qd[k]);
+          st_w(a.QDot + off, dq);
+        }
       }
       if (a.resid)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) s.mx[k][tid] = nanmax(s.mx[k][tid], fabs(double(qd[k])));
+        for (int k = 0; k < W; ++k) mx[k] = nanmax(mx[k], fabs(double(qd[k])));
       if (a.update) {
-        real gn[4];
-        if (a.first) {
+        double q[W] = {};
+        if (on) {
+          real gn[W];
+          if (a.first) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) gn[k] = real(a.b) * qd[k];
-        } else {
-          ld4(&in.G[m * 4], gn);
+            for (int k = 0; k < W; ++k) gn[k] = real(a.b) * qd[k];
+          } else {
+            ld_w(&in.G[m * 4 + h], gn);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) gn[k] = real(a.a) * gn[k] + real(a.b) * qd[k];
+            for (int k = 0; k < W; ++k) gn[k] = real(a.a) * gn[k] + real(a.b) * qd[k];
+          }
+          st_w(a.G + off, gn);
+          ld_w(&in.Q[m * 4 + h], q);
+#pragma unroll
+          for (int k = 0; k < W; ++k) q[k] = q[k] + a.c * double(gn[k]);
+          st_w(a.Q + off, q);
+          real r[W];
+#pragma unroll
+          for (int k = 0; k < W; ++k) r[k] = real(q[k]);
+          if (LGL) {
+            real* tp = a.T_out + size_t(e0 + le) * FT * 4 + h;
+            if (j == 0) st_w(tp + i * 4, r);
+            if (i == P - 1) st_w(tp + (P + j) * 4, r);
+            if (j == P - 1) st_w(tp + (2 * P + i) * 4, r);
+            if (i == 0) st_w(tp + (3 * P + j) * 4, r);
+          } else {
+#pragma unroll
+            for (int k = 0; k < W; ++k) s.Fc[(h + k) * VS + o] = r[k];
+          }
         }
-        st4(a.G + off, gn);
-        double q[4];
-        ld4(&in.Q[m * 4], q);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) q[k] = q[k] + a.c * double(gn[k]);
-        st4(a.Q + off, q);
-        check_state(a.health, a.health_host, q[0], q[1], q[2], q[3], e0 + le);
-        const real r[4] = {real(q[0]), real(q[1]), real(q[2]), real(q[3])};
-        if (LGL) {
-          real* tp = a.T_out + size_t(e0 + le) * FT * 4;
-          if (j == 0) st4(tp + i * 4, r);
-          if (i == P - 1) st4(tp + (P + j) * 4, r);
-          if (j == P - 1) st4(tp + (2 * P + i) * 4, r);
-          if (i == 0) st4(tp + (3 * P + j) * 4, r);
+        if constexpr (W == 2) {   // the pair's other half, for the check of the whole state
+          const double r0 = __shfl_xor_sync(0xffffffffu, q[0], 1), r1 = __shfl_xor_sync(0xffffffffu, q[1], 1);
+          if (on && h == 0) check_state(a.health, a.health_host, q[0], q[1], r0, r1, e0 + le);
         } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) s.Fc[k * VS + o] = r[k];
+          if (on) check_state(a.health, a.health_host, q[0], q[1], q[2], q[3], e0 + le);
         }
       }
     }
@@ -492,14 +538,8 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     b ^= 1;
     slot = next_slot;
   }
-  if (a.resid) {
-    __syncthreads();
-    if (tid < 4) {
-      double m = 0.0;
-      for (int t = 0; t < T; ++t) m = nanmax(m, s.mx[tid][t]);
-      a.resid[size_t(blockIdx.x) * 4 + tid] = m;
-    }
-  }
+  if (a.resid) residual_partial<W, T>(mx, reinterpret_cast<double*>(s.in), a.resid + size_t(blockIdx.x) * 4, tid);
+  static_assert(sizeof(s.in) >= W * T * sizeof(double), "scratch of the residual maxima");
 }
 
 // Traces of the resident state (after hg_set_state).
