@@ -123,13 +123,14 @@ static void health_check(hg_ctx* c) {
 // leave half of the SMs or more without one (fewer than two groups per SM): there a stage is one pass of
 // latency, and the smaller groups spread it over the chip.
 // (Navier-Stokes orders 9 and 10 run one element per group in both variants, one instantiation.)
+static bool in_double(const hg_ctx* c) { return c->precision == HG_PREC_FP64; }
 static int stage_variant(const hg_ctx* c, int variant) {
   if (c->ns && c->P >= 10) return 0;
-  return variant || c->n_el < 2 * c->n_sm * (c->ns ? epb_ns_of(c->P, 0) : epb_stage(c->P, 0)) ? 1 : 0;
+  return variant || c->n_el < 2 * c->n_sm * (c->ns ? epb_ns_of(c->P, 0, in_double(c)) : epb_stage(c->P, 0)) ? 1 : 0;
 }
 static int epb_of(const hg_ctx* c, int variant) {
   const int v = stage_variant(c, variant);
-  return c->ns ? epb_ns_of(c->P, v) : epb_stage(c->P, v);
+  return c->ns ? epb_ns_of(c->P, v, in_double(c)) : epb_stage(c->P, v);
 }
 // per-CTA residual partials
 static int max_grid(const hg_ctx* c) { return std::min(c->n_el, 32 * c->n_sm); }
@@ -1583,7 +1584,7 @@ extern "C" int hg_get_tiling(const hg_ctx* c, int32_t out[3]) {
   out[0] = c->tiling;
   out[1] = epb;
   const int v = stage_variant(c, c->tiling);
-  out[2] = c->ns ? ns_threads(c->P, v) : stage_threads(c->P, v);
+  out[2] = c->ns ? ns_threads(c->P, v, in_double(c)) : stage_threads(c->P, v);
   return 0;
 }
 

@@ -184,7 +184,7 @@ void launch_ns_PV(hg_ctx* c, const NSArgs<real>& a) {
 // evaluated whenever weights are set.
 template <int P, typename real>
 struct SensorTiles {
-  static constexpr int EPB = epb_ns(P), T = ns_threads(P, 0), V0 = EPB * P * (P | 1);
+  static constexpr int EPB = epb_ns(P, sizeof(real) == 8), T = ns_threads(P, 0, sizeof(real) == 8), V0 = EPB * P * (P | 1);
   static constexpr int VM = sizeof(real) == 8 ? 16 : 32, VS = V0 + (VM + VM / 4 - V0 % VM) % VM;
   alignas(16) real Q[4 * VS];
   real U[2 * VS];
@@ -194,7 +194,7 @@ struct SensorTiles {
 template <int P, typename real>
 struct SensorOps { real Vinv[P * P]; };
 template <int P, typename real>
-__global__ void __launch_bounds__(ns_threads(P, 0)) sensor_eval_kernel(int n_el, const double* Q, const __grid_constant__ SensorOps<P, real> op,
+__global__ void __launch_bounds__(ns_threads(P, 0, sizeof(real) == 8)) sensor_eval_kernel(int n_el, const double* Q, const __grid_constant__ SensorOps<P, real> op,
                                                                        SensorArgs sa, PhysConst pc, float* feat,
                                                                        double* out) {
   using Tl = SensorTiles<P, real>;

@@ -79,12 +79,16 @@ struct NSArgs {
   int* health_host;         // mapped host flag set beside it
 };
 
-// Elements per group and threads per CTA: variant 0, and variant 1 for small meshes.
-__host__ __device__ constexpr int epb_ns(int P) { return P == 2 ? 16 : P <= 4 ? 8 : P <= 6 ? 4 : P <= 8 ? 2 : 1; }
+// Elements per group and threads per CTA: variant 0, and variant 1 for small meshes.  At order 5 a double group is
+// half a float one: a CTA's shared memory then lets five reside on an SM instead of two (stage and gradient on the
+// cylinder mesh 58.5 -> 56.4 us, with the jumps indicator 36.3 -> 32.9; in float 33.5 against 34.6).
+__host__ __device__ constexpr int epb_ns(int P, bool dbl) {
+  return P == 2 ? 16 : P <= 4 ? 8 : P == 5 ? 4 : P == 6 ? (dbl ? 2 : 4) : P <= 8 ? 2 : 1;
+}
 __host__ __device__ constexpr int epb_ns_small(int P) { return P <= 3 ? 4 : P <= 6 ? 2 : 1; }
-__host__ __device__ constexpr int epb_ns_of(int P, int variant) { return variant ? epb_ns_small(P) : epb_ns(P); }
-__host__ __device__ constexpr int ns_threads(int P, int variant) {
-  return (cmax(P * P, 4 * P) * epb_ns_of(P, variant) + 31) / 32 * 32;
+__host__ __device__ constexpr int epb_ns_of(int P, int variant, bool dbl) { return variant ? epb_ns_small(P) : epb_ns(P, dbl); }
+__host__ __device__ constexpr int ns_threads(int P, int variant, bool dbl) {
+  return (cmax(P * P, 4 * P) * epb_ns_of(P, variant, dbl) + 31) / 32 * 32;
 }
 
 // Nodal operators, passed by value (constant bank); dl = lb^T D, the normal derivatives at the sides.
@@ -135,7 +139,7 @@ __device__ __forceinline__ void store_line(real* u, const int st, const real (&v
 // Shared memory of a CTA.  GRAD: the gradient kernel's (no RK register, no stored gradient to read).
 template <int P, int V, typename real, bool AFFINE, bool IP, bool AV, bool VISC, bool GRAD>
 struct NSTiles {
-  static constexpr int EPB = epb_ns_of(P, V), T = ns_threads(P, V);
+  static constexpr int EPB = epb_ns_of(P, V, sizeof(real) == 8), T = ns_threads(P, V, sizeof(real) == 8);
   static constexpr int NP = P * P, FT = 4 * P, PO = P | 1, NN = EPB * NP, NF = EPB * FT, GS = vol_geo_stride(P, AFFINE);
   static constexpr int VM = sizeof(real) == 8 ? 16 : 32, V0 = EPB * P * PO;
   static constexpr int VS = V0 + (VM + VM / 4 - V0 % VM) % VM;   // = VM / 4 modulo VM
@@ -521,7 +525,7 @@ __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSAr
 // resident state.  Then the modal or learned indicator, on the first stage of a time step (and for a bare
 // time derivative); the later stages of the step keep that viscosity.
 template <int P, int V, typename real, bool AFFINE, bool IP, bool AV>
-__global__ void __launch_bounds__(ns_threads(P, V))
+__global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
     ns_gradient_kernel(const __grid_constant__ NSArgs<real> a, const __grid_constant__ NSOps<P, real> op) {
   using Tl = NSTiles<P, V, real, AFFINE, IP, AV, true, true>;
   constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, PO = Tl::PO, VS = Tl::VS, GS = Tl::GS, NF = Tl::NF,
@@ -852,7 +856,7 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
 //   E  nodes: 1/J, RK update, health check;
 //   F  lines: traces of the new state and, on the fused path, of its gradient; then its indicator.
 template <int P, int V, typename real, bool AFFINE, bool IP, bool AV, bool VISC>
-__global__ void __launch_bounds__(ns_threads(P, V), ns_min_ctas<NSTiles<P, V, real, AFFINE, IP, AV, VISC, false>>())
+__global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ctas<NSTiles<P, V, real, AFFINE, IP, AV, VISC, false>>())
     ns_stage_kernel(const __grid_constant__ NSArgs<real> a, const __grid_constant__ NSOps<P, real> op) {
   using Tl = NSTiles<P, V, real, AFFINE, IP, AV, VISC, false>;
   constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, PO = Tl::PO, VS = Tl::VS, GS = Tl::GS, NF = Tl::NF,
@@ -880,14 +884,14 @@ __global__ void __launch_bounds__(ns_threads(P, V), ns_min_ctas<NSTiles<P, V, re
     if (AV && !local && a.av == 1)
       for (int le = 0; le < n_act; ++le) local = local || in.mu[le] != 0.0;
 
-    // A
-    constexpr int NFR = (NF + 31) / 32 * 32;
-    for (int x = tid; x < NFR + Tl::NN; x += T) {
-      if (x < NFR) {
-        if (x < n_act * FT) ns_face_task<P, Tl, real, AFFINE, IP, AV, VISC>(a, ph, s, in, side, x, e0);
-      } else {
-        const int m = x - NFR, le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
-        if (le >= n_act) continue;
+    // A.  Where the face nodes leave whole warps over, those take all volume nodes (a face task is three times as
+    // long as a node's); else every warp does its faces, then its nodes.
+    constexpr int NFR = (NF + 31) / 32 * 32, NT = T > NFR ? T - NFR : T;
+    static_assert(NFR <= T, "one round of face tasks");
+    if (tid < n_act * FT) ns_face_task<P, Tl, real, AFFINE, IP, AV, VISC>(a, ph, s, in, side, tid, e0);
+    if (T == NFR || tid >= NFR) {
+      for (int m = T == NFR ? tid : tid - NFR; m < n_act * NP; m += NT) {
+        const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
         double qd[4];
         ld4(&s.state(b)[m * 4], qd);
         const real q[4] = {real(qd[0]), real(qd[1]), real(qd[2]), real(qd[3])};
