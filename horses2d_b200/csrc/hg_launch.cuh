@@ -6,14 +6,15 @@
 #include <algorithm>
 #include <atomic>
 
-// Resident CTAs per SM of a persistent kernel with `smem` bytes of dynamic shared memory, after allowing it
-// that much; looked up once per kernel and device.
+// Resident CTAs per SM of a persistent kernel with `smem` bytes of dynamic shared memory; looked up once per kernel,
+// size and device.  `most` is the largest size that any launch of the kernel uses: the attribute holds for all of
+// them, so that it must not be lowered by a launch that needs less.
 template <typename K>
-static int resident_ctas(const hg_ctx* c, std::atomic<int>* known, K kernel, int threads, size_t smem) {
+static int resident_ctas(const hg_ctx* c, std::atomic<int>* known, K kernel, int threads, size_t smem, size_t most) {
   std::atomic<int>* slot = c->device < HG_KNOWN_DEVICES ? &known[c->device] : nullptr;
   int n = slot ? slot->load(std::memory_order_relaxed) : 0;
   if (n > 0) return n;
-  HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)));
   max_carveout(kernel);
   HG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
   if (n < 1) throw std::runtime_error("stage kernel does not fit on this device");
@@ -34,8 +35,13 @@ static void launch_dependent(hg_ctx* c, void (*kernel)(KA...), int grid, int thr
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = c->prof ? 0 : 1;
-  HG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  // (the default streams keep plain launches: their ordering against other streams is their own)
+  cfg.numAttrs = c->prof || reinterpret_cast<uintptr_t>(c->stream) <= uintptr_t(2) ? 0 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // reported here: not left behind for the next call
+    throw std::runtime_error(std::string("stage kernel launch: ") + cudaGetErrorString(e));
+  }
 }
 
 template <int P, typename real>
@@ -58,7 +64,7 @@ static void launch_stage_PAL(hg_ctx* c, const StageArgs<real>& a) {
   using Tl = StageTiles<P, V, real, AFFINE, LGL>;
   static std::atomic<int> known[HG_KNOWN_DEVICES];
   const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
-  const int most = c->n_sm * std::min(32, resident_ctas(c, known, stage_kernel<P, V, real, AFFINE, LGL>, Tl::T, sizeof(Tl)));
+  const int most = c->n_sm * std::min(32, resident_ctas(c, known, stage_kernel<P, V, real, AFFINE, LGL>, Tl::T, sizeof(Tl), sizeof(Tl)));
   // every CTA takes the same number of groups but the last ones: no more CTAs than that needs
   const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
   if (a.resid) c->n_resid = grid;
@@ -122,7 +128,7 @@ static int launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind,
   static_assert(sizeof(Tl) + MLP_BYTES <= 227 * 1024, "shared memory of a CTA");
   const size_t smem = sizeof(Tl) + (weights ? MLP_BYTES : 0);
   const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
-  const int most = c->n_sm * std::min(32, resident_ctas(c, known, kernel, Tl::T, smem));
+  const int most = c->n_sm * std::min(32, resident_ctas(c, known, kernel, Tl::T, smem, sizeof(Tl) + MLP_BYTES));
   const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
   timed(c, kind, [&] { launch_dependent(c, kernel, grid, Tl::T, smem, a, op); });
   ++c->launches;
@@ -231,7 +237,7 @@ template <int P, typename real>
 void launch_sensor_eval_P(hg_ctx* c, float* feat, double* out) {
   using Tl = SensorTiles<P, real>;
   static std::atomic<int> known[HG_KNOWN_DEVICES];
-  resident_ctas(c, known, sensor_eval_kernel<P, real>, Tl::T, sizeof(Tl));   // allows the shared memory
+  resident_ctas(c, known, sensor_eval_kernel<P, real>, Tl::T, sizeof(Tl), sizeof(Tl));   // allows the shared memory
   SensorOps<P, real> op;
   const double* vinv = c->h_mats.data() + 2 * P * P + 7 * P;
   for (int k = 0; k < P * P; ++k) op.Vinv[k] = real(vinv[k]);

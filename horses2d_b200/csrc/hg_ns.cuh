@@ -26,7 +26,10 @@
 // nodes of a (variable, line) in registers and takes the operator from the constant bank.  The kernels before
 // held one node per thread and read the operators and the tiles from shared memory, 1.25 loads per
 // multiply-add: their shared-memory pipe ran at 78-81 % of its peak at N = 7 with a quarter of the FP64 rate
-// used, and a third of the warps' time went into global loads at the phase that needed them.
+// used, and a third of the warps' time went into global loads at the phase that needed them.  Measured per stage
+// (then -> now): shear layer 384 x 384 N = 7 SIPG FP64 1.57 -> 1.10 ms, FP32 0.81 -> 0.65 ms; cylinder 64 x 128 N = 5
+// BR1 FP64 90 -> 57 us, FP32 54 -> 34 us; shock 512 x 64 N = 3 FP64 62 -> 51 us, FP32 35 -> 32 us.  What bounds them
+// now: the chain of a face task (700 instructions in double) at 12 to 24 warps per SM, and barriers.
 #pragma once
 #include "hg_stage.cuh"
 #include "hg_sensor.cuh"

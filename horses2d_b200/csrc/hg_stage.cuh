@@ -18,10 +18,12 @@
 //      Q += c G (DGTimeIntegrator.f90:282-365); Gauss-Lobatto: the boundary nodes are the new traces;
 //   D  Legendre-Gauss: one thread per (variable, line): the traces of the new state at the line's ends
 //      (interpolateSolutionToBoundaries, :1520-1574) for the next launch (ping-pong buffer).
-// What bounds it: instruction issue and HBM.  One thread per node with its loads where they were used (the
-// form before) spent half of its warps' cycles on global loads and filled 62 % of the lanes of its face
-// phase; measured with 512 x 512 elements, N = 4, Gauss-Lobatto, FP64: 0.80 ms a stage then, 0.32 ms now
-// (1.17 GB of state, register and trace traffic: 3.7 TB/s); 16 x 16 elements: 20.5 -> 14.3 us a step.
+// What bounds it: latency, with 15 warps per SM in double (registers and shared memory), then the shared-memory
+// pipe (58 %); in float instruction issue (70 %).  One thread per node with its loads where they were used (the form
+// before) spent half of its warps' cycles on global loads and filled 62 % of the lanes of its face phase; measured
+// with 512 x 512 elements, N = 4, Gauss-Lobatto, FP64: 0.80 ms a stage then, 0.31 ms now (1.17 GB of state, register
+// and trace traffic: 3.8 TB/s); 16 x 16 elements: 20.5 -> 10.8 us a step.  Fewer or more elements to a group (4, 6)
+// and 96 to 256 threads came out between equal and 25 % slower at N = 4.
 // The Riemann flux of an interior face is evaluated by both of its elements with identical arguments
 // (LEFT trace, RIGHT trace, LEFT's normal), so both see the same value and the face needs no separate
 // launch or flux buffer.

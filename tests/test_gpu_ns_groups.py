@@ -71,3 +71,21 @@ def test_stepped_and_loaded_states_agree(N, precision):
     g.time_steps(hg.SCHEME_RK3, 2, 0.0, dt)
     h.time_steps(hg.SCHEME_RK3, 2, 0.0, dt)
     assert np.array_equal(g.state(), h.state())
+
+
+def test_sensor_kinds_take_turns_in_one_process():
+    """Learned, modal, learned contexts of one order and precision: the learned ones launch the same kernels with the
+    network's weights in shared memory, whatever ran in between."""
+    from test_gpu_sensor import random_problem
+    p, _, _, _ = random_problem(1, 7)
+    states = []
+    for kind in (hg.SENSOR_LEARNED, hg.SENSOR_MODAL, hg.SENSOR_LEARNED):
+        for viscous in (O.IP, O.BR1):
+            orc, g, Q = box(9, 7, 3, viscous, True, hg.PREC_FP32)
+            if kind == hg.SENSOR_LEARNED:
+                g.set_sensor(kind, mlp=p)
+            g.set_state(Q)
+            g.time_steps(hg.SCHEME_RK3, 2, 0.0, 1e-7)
+            states.append(g.state())
+    assert all(np.isfinite(s).all() for s in states)
+    assert np.array_equal(states[0], states[4]) and np.array_equal(states[1], states[5])
