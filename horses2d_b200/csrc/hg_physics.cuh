@@ -39,23 +39,9 @@ template <typename real> __device__ __forceinline__ real pow_r(real x, real y);
 template <> __device__ __forceinline__ double pow_r(double x, double y) { return pow(x, y); }
 template <> __device__ __forceinline__ float pow_r(float x, float y) { return powf(x, y); }
 
-// 1 / rho and sqrt(rho) of a face state.  In double one reciprocal square root gives both (the division and
-// the square root are instruction sequences of their own there: a Roe flux took five and three of them,
-// two thirds of its instructions); in float they are one special-function operation each, and the
-// reciprocal keeps its own rounding.  A negative density gives NaN in either.
-struct RootsD { double inv, root; };
-struct RootsF { float inv, root; };
-__device__ __forceinline__ RootsD density_roots(double rho) {
-  const double r = rsqrt(rho);
-  return {r * r, rho * r};
-}
-__device__ __forceinline__ RootsF density_roots(float rho) { return {1.0f / rho, sqrtf(rho)}; }
-__device__ __forceinline__ double rsqrt_r(double x) { return rsqrt(x); }
-__device__ __forceinline__ float rsqrt_r(float x) { return rsqrtf(x); }
-
 template <typename real>
 __device__ __forceinline__ void inviscid_flux(const Phys<real>& ph, const real* u, real* f, real* g) {
-  const real invRho = density_roots(u[0]).inv;
+  const real invRho = real(1) / u[0];
   const real vx = u[1] * invRho, vy = u[2] * invRho;
   const real p = ph.gm1 * (u[3] - real(0.5) * u[1] * vx - real(0.5) * u[2] * vy);
   f[0] = u[1]; f[1] = u[1] * vx + p; f[2] = u[1] * vy; f[3] = (u[3] + p) * vx;
@@ -80,28 +66,23 @@ __device__ __forceinline__ void rotate_back_scale(const Phys<real>& ph, real* F,
 
 template <typename real>
 __device__ __forceinline__ void roe(const Phys<real>& ph, const real* qL, const real* qR, real nx, real ny, real* F) {
-  const auto tL = density_roots(qL[0]), tR = density_roots(qR[0]);
-  const real rhoL = qL[0];
-  const real uL = (qL[1] * nx + qL[2] * ny) * tL.inv, vL = (-qL[1] * ny + qL[2] * nx) * tL.inv;
-  const real kL = real(0.5) * (uL * uL + vL * vL);
-  const real pL = ph.gm1 * (qL[3] - rhoL * kL);
-  const real HL = ph.cp * pL * tL.inv + kL;
-  const real rhoR = qR[0];
-  const real uR = (qR[1] * nx + qR[2] * ny) * tR.inv, vR = (-qR[1] * ny + qR[2] * nx) * tR.inv;
-  const real kR = real(0.5) * (uR * uR + vR * vR);
-  const real pR = ph.gm1 * (qR[3] - rhoR * kR);
-  const real HR = ph.cp * pR * tR.inv + kR;
-  const real invrho = real(1) / (tL.root + tR.root);
-  const real u = (tL.root * uL + tR.root * uR) * invrho;
-  const real v = (tL.root * vL + tR.root * vR) * invrho;
-  const real H = (tL.root * HL + tR.root * HR) * invrho;
-  const real k = real(0.5) * (u * u + v * v);
-  const real a2 = ph.gm1 * (H - k);
-  const real ia = rsqrt_r(a2), a = a2 * ia;   // one root for a, 1/a and 1/a^2
+  const real rhoL = qL[0], invRhoL = real(1) / rhoL, sqrtRhoL = sqrt_r(rhoL);
+  const real uL = (qL[1] * nx + qL[2] * ny) * invRhoL, vL = (-qL[1] * ny + qL[2] * nx) * invRhoL;
+  const real pL = ph.gm1 * (qL[3] - real(0.5) * rhoL * (uL * uL + vL * vL));
+  const real HL = ph.cp * pL * invRhoL + real(0.5) * (uL * uL + vL * vL);
+  const real rhoR = qR[0], invRhoR = real(1) / rhoR, sqrtRhoR = sqrt_r(rhoR);
+  const real uR = (qR[1] * nx + qR[2] * ny) * invRhoR, vR = (-qR[1] * ny + qR[2] * nx) * invRhoR;
+  const real pR = ph.gm1 * (qR[3] - real(0.5) * rhoR * (uR * uR + vR * vR));
+  const real HR = ph.cp * pR * invRhoR + real(0.5) * (uR * uR + vR * vR);
+  const real invrho = real(1) / (sqrtRhoL + sqrtRhoR);
+  const real u = (sqrtRhoL * uL + sqrtRhoR * uR) * invrho;
+  const real v = (sqrtRhoL * vL + sqrtRhoR * vR) * invrho;
+  const real H = (sqrtRhoL * HL + sqrtRhoR * HR) * invrho;
+  const real a = sqrt_r(ph.gm1 * (H - real(0.5) * (u * u + v * v)));
   const real dq0 = rhoR - rhoL, dq1 = rhoR * uR - rhoL * uL, dq2 = rhoR * vR - rhoL * vL, dq3 = qR[3] - qL[3];
   const real al2 = dq2 - v * dq0;
-  const real al1 = ph.gm1 * (dq0 * (H - u * u) + u * dq1 - dq3 + al2 * v) * (ia * ia);
-  const real al0 = (dq0 * (u + a) - dq1 - a * al1) * (real(0.5) * ia);
+  const real al1 = ph.gm1 * (dq0 * (H - u * u) + u * dq1 - dq3 + (dq2 - v * dq0) * v) / (a * a);
+  const real al0 = (dq0 * (u + a) - dq1 - a * al1) / (real(2) * a);
   const real al3 = dq0 - (al0 + al1);
   flux_normal(rhoL, uL, vL, pL, HL, F);
   // waves with negative speed, added in the reference's order (u-a, u, u, u+a)
@@ -110,7 +91,7 @@ __device__ __forceinline__ void roe(const Phys<real>& ph, const real* qL, const 
     F[0] += s; F[1] += s * (u - a); F[2] += s * v; F[3] += s * (H - u * a);
     if (!(u > real(0))) {
       const real s1 = al1 * u;
-      F[0] += s1; F[1] += s1 * u; F[2] += s1 * v; F[3] += s1 * k;
+      F[0] += s1; F[1] += s1 * u; F[2] += s1 * v; F[3] += s1 * (real(0.5) * (u * u + v * v));
       const real s2 = al2 * u;
       F[2] += s2; F[3] += s2 * v;
       if (!(u + a > real(0))) {
@@ -124,33 +105,31 @@ __device__ __forceinline__ void roe(const Phys<real>& ph, const real* qL, const 
 
 template <typename real>
 __device__ __forceinline__ void hll(const Phys<real>& ph, const real* qL, const real* qR, real nx, real ny, real* F) {
-  const auto tL = density_roots(qL[0]), tR = density_roots(qR[0]);
-  const real rhoL = qL[0], rhoeL = qL[3];
-  const real uL = (qL[1] * nx + qL[2] * ny) * tL.inv, vL = (-qL[1] * ny + qL[2] * nx) * tL.inv;
-  const real kL = real(0.5) * (uL * uL + vL * vL);
-  const real pL = ph.gm1 * (qL[3] - rhoL * kL);
-  const real HL = ph.cp * pL * tL.inv + kL;
-  const real aL = sqrt_r(ph.gamma * pL * tL.inv);
-  const real rhoR = qR[0], rhoeR = qR[3];
-  const real uR = (qR[1] * nx + qR[2] * ny) * tR.inv, vR = (-qR[1] * ny + qR[2] * nx) * tR.inv;
-  const real kR = real(0.5) * (uR * uR + vR * vR);
-  const real pR = ph.gm1 * (qR[3] - rhoR * kR);
-  const real HR = ph.cp * pR * tR.inv + kR;
-  const real aR = sqrt_r(ph.gamma * pR * tR.inv);
-  const real invrho = real(1) / (tL.root + tR.root);
-  const real u = (tL.root * uL + tR.root * uR) * invrho;
-  const real v = (tL.root * vL + tR.root * vR) * invrho;
-  const real H = (tL.root * HL + tR.root * HR) * invrho;
+  const real rhoL = qL[0], invRhoL = real(1) / rhoL;
+  const real uL = (qL[1] * nx + qL[2] * ny) * invRhoL, vL = (-qL[1] * ny + qL[2] * nx) * invRhoL;
+  const real pL = ph.gm1 * (qL[3] - real(0.5) * rhoL * (uL * uL + vL * vL));
+  const real HL = ph.cp * pL * invRhoL + real(0.5) * (uL * uL + vL * vL);
+  const real aL = sqrt_r(ph.gamma * pL * invRhoL), rhoeL = qL[3];
+  const real rhoR = qR[0], invRhoR = real(1) / rhoR;
+  const real uR = (qR[1] * nx + qR[2] * ny) * invRhoR, vR = (-qR[1] * ny + qR[2] * nx) * invRhoR;
+  const real pR = ph.gm1 * (qR[3] - real(0.5) * rhoR * (uR * uR + vR * vR));
+  const real HR = ph.cp * pR * invRhoR + real(0.5) * (uR * uR + vR * vR);
+  const real aR = sqrt_r(ph.gamma * pR * invRhoR), rhoeR = qR[3];
+  const real sqrtRhoL = sqrt_r(rhoL), sqrtRhoR = sqrt_r(rhoR);
+  const real invrho = real(1) / (sqrtRhoL + sqrtRhoR);
+  const real u = (sqrtRhoL * uL + sqrtRhoR * uR) * invrho;
+  const real v = (sqrtRhoL * vL + sqrtRhoR * vR) * invrho;
+  const real H = (sqrtRhoL * HL + sqrtRhoR * HR) * invrho;
   const real a = sqrt_r(ph.gm1 * (H - real(0.5) * (u * u + v * v)));
   const real SL = fmin(uL - aL, u - a), SR = fmax(uR + aR, u + a);
   if (SL >= real(0)) flux_normal(rhoL, uL, vL, pL, HL, F);
   else if (SR <= real(0)) flux_normal(rhoR, uR, vR, pR, HR, F);
   else {
-    const real invdS = real(1) / (SR - SL), mL = rhoL * uL, mR = rhoR * uR, S2 = SL * SR;
-    F[0] = (SR * mL - SL * mR + S2 * (rhoR - rhoL)) * invdS;
-    F[1] = (SR * (mL * uL + pL) - SL * (mR * uR + pR) + S2 * (mR - mL)) * invdS;
-    F[2] = (SR * mL * vL - SL * mR * vR + S2 * (rhoR * vR - rhoL * vL)) * invdS;
-    F[3] = (SR * mL * HL - SL * mR * HR + S2 * (rhoeR - rhoeL)) * invdS;
+    const real invdS = real(1) / (SR - SL);
+    F[0] = (SR * rhoL * uL - SL * rhoR * uR + SL * SR * (rhoR - rhoL)) * invdS;
+    F[1] = (SR * (rhoL * uL * uL + pL) - SL * (rhoR * uR * uR + pR) + SL * SR * (rhoR * uR - rhoL * uL)) * invdS;
+    F[2] = (SR * rhoL * uL * vL - SL * rhoR * uR * vR + SR * SL * (rhoR * vR - rhoL * vL)) * invdS;
+    F[3] = (SR * uL * rhoL * HL - SL * uR * rhoR * HR + SR * SL * (rhoeR - rhoeL)) * invdS;
   }
   rotate_back_scale(ph, F, nx, ny);
 }
@@ -335,7 +314,7 @@ __device__ __forceinline__ void euler_wall_flux(const Phys<real>& ph, const real
 template <typename real>
 __device__ __forceinline__ void viscous_flux(const Phys<real>& ph, const real* q, const real* dqx, const real* dqy,
                                              real* Fx, real* Fy) {
-  const real invRho = density_roots(q[0]).inv;   // shared with the Riemann solver's at a face node
+  const real invRho = real(1) / q[0];
   const real u = q[1] * invRho, v = q[2] * invRho;
   const real uDivRho = u * invRho, vDivRho = v * invRho;
   const real divV = -uDivRho * dqx[0] + invRho * dqx[1] - vDivRho * dqy[0] + invRho * dqy[2];
@@ -355,7 +334,7 @@ __device__ __forceinline__ void viscous_flux(const Phys<real>& ph, const real* q
 template <typename real>
 __device__ __forceinline__ void viscous_flux_adiabatic(const Phys<real>& ph, const real* q, const real* qB,
                                                        const real* dqx, const real* dqy, real* Fx, real* Fy) {
-  const real invRho = density_roots(q[0]).inv;
+  const real invRho = real(1) / q[0];
   const real u = q[1] * invRho, v = q[2] * invRho;
   const real uDivRho = u * invRho, vDivRho = v * invRho;
   const real divV = -uDivRho * dqx[0] + invRho * dqx[1] - vDivRho * dqy[0] + invRho * dqy[2];
