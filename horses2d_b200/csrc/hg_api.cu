@@ -53,7 +53,7 @@ void ctx_free(hg_ctx* c) {
   drop_graph(c);
   for (cudaEvent_t e : c->prof_pool) cudaEventDestroy(e);
   void* ptrs[] = {c->d_side, c->d_side_geo, c->d_vol_geo, c->d_mats, c->d_zones, c->d_Q, c->d_G, c->d_T[0], c->d_T[1],
-                  c->d_QDot, c->d_resid, c->d_resid_out, c->d_elmax, c->d_side_invh, c->d_face_metric, c->d_GT[0],
+                  c->d_QDot, c->d_resid, c->d_resid_out, c->d_elmax, c->d_side_invh, c->d_jac, c->d_face_metric, c->d_GT[0],
                   c->d_GT[1], c->d_av_el, c->d_side_area, c->d_mu_av[0], c->d_mu_av[1], c->d_mlp, c->d_feat_lo,
                   c->d_feat_hi, c->d_dQ,
                   c->d_FX, c->d_bq, c->d_si_out, c->d_NF, c->d_NFG, c->d_NJ, c->d_exact_sides};
@@ -206,6 +206,7 @@ static void run_ns_stage(hg_ctx* c, double ca, double cb, double cc, bool first,
   a.side_geo = static_cast<const real*>(c->d_side_geo);
   a.side_invh = c->d_side_invh;
   a.vol_geo = static_cast<const real*>(c->d_vol_geo);
+  a.jac = static_cast<const real*>(c->d_jac);
   a.face_metric = static_cast<const real*>(c->d_face_metric);
   a.zones = c->d_zones;
   a.bq = c->d_bq;
@@ -678,6 +679,7 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
     for (auto& g_ : c->d_GT) g_ = dalloc<char>(size_t(E) * 4 * P * 8 * rs);
     c->d_dQ = dalloc<char>(size_t(c->ndof) * 2 * rs);
     HG_CUDA(cudaMemcpy(c->d_side_invh, sinvh.data(), sinvh.size() * sizeof(double), cudaMemcpyHostToDevice));
+    if (!c->affine && !c->ip && c->precision == HG_PREC_FP32) upload_real(c->d_jac, m->jac, size_t(E) * NP);
     if (!c->affine && c->grad_faces) {
       // metrics over the jacobian at the side nodes, both interpolated along the normal line
       std::vector<double> fm(size_t(E) * 4 * P * 4);

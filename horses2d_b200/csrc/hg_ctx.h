@@ -60,6 +60,7 @@ struct hg_ctx {
   float* d_mlp = nullptr;
   float* d_feat_lo = nullptr;
   float* d_feat_hi = nullptr;
+  void* d_jac = nullptr;          // [n_el][NP] J (curved BR1 in FP32)
   void* d_face_metric = nullptr;  // [n_el*4][P][4] Ja/J at the side nodes (curved, gradient faces), context precision
   void* d_GT[2] = {nullptr, nullptr};   // gradient traces [n_el*4][P][2][4] per trace parity (as d_T)
   void* d_dQ = nullptr;           // element gradients [n_el][2][4][NP] (Navier-Stokes)

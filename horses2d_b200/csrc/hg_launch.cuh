@@ -90,8 +90,7 @@ void launch_trace_P(hg_ctx* c) {
   timed(c, HG_KERNEL_TRACE, [&] {
     trace_kernel<P, EPB, real><<<grid, block_for(P), 0, c->stream>>>(c->n_el, c->d_Q, c->d_mats,
                                                                      static_cast<real*>(c->d_T[c->cur]),
-                                                                     c->ns ? (c->ip ? TRACE_PLAIN : TRACE_RELATIVE)
-                                                                           : c->node_type == HG_NODES_LGL ? TRACE_NODAL : TRACE_PLAIN);
+                                                                     !c->ns && c->node_type == HG_NODES_LGL);
   });
   ++c->launches;
 }

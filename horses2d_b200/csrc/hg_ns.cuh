@@ -43,6 +43,7 @@ struct NSArgs {
   const real* side_geo;     // normals / dS (per node, or per side when AFFINE)
   const double* side_invh;  // [n_el*4] invh of the side's edge
   const real* vol_geo;      // element records of vol_geo_stride reals (hg_stage.cuh)
+  const real* jac;          // [n_el][P*P] J (curved BR1 in float)
   const real* face_metric;  // [n_el*4][P][4] Ja00/J Ja01/J Ja10/J Ja11/J at the side nodes (curved, gradient faces)
   const Zone* zones;
   const double* bq;         // per-node Dirichlet states [rows][P][4] (sides whose side.w >= 0)
@@ -118,16 +119,6 @@ __device__ __forceinline__ real dot(const real* c, const real (&in)[P]) {
   for (int l = 0; l < P; ++l) r += c[l] * in[l];
   return r;
 }
-// The state's trace at an end of a line (boundary interpolant c, which sums to 1) for BR1.  In float relative to
-// the line's first node, so that the products round a difference; trace_kernel sums the same way.
-template <int P, typename real>
-__device__ __forceinline__ real trace_dot(const real* c, const real (&in)[P]) {
-  if (sizeof(real) == 8) return dot<P>(c, in);
-  real r = real(0);
-#pragma unroll
-  for (int l = 1; l < P; ++l) r += c[l] * (in[l] - in[0]);
-  return in[0] + r;
-}
 template <int P, typename real>
 __device__ __forceinline__ void load_line(const real* u, const int st, real (&in)[P]) {
 #pragma unroll
@@ -180,7 +171,10 @@ struct NSTiles {
   // their contractions
   alignas(16) real Q[4 * VS];
   real Fc[4 * VS], Gc[4 * VS];
-  real X[GRAD && !IP ? 4 * VS : 4], Y[GRAD && !IP ? 4 * VS : 4];   // BR1 volume terms of the second direction
+  static constexpr bool SUMS = !IP && SumOps<P, real>::ON;   // BR1 in float: a node's sums in one order (hg_stage.cuh)
+  // BR1 volume terms of the second direction
+  real X[GRAD && !IP && !SUMS ? 4 * VS : 4], Y[GRAD && !IP && !SUMS ? 4 * VS : 4];
+  SumOps<P, real, SUMS> sum;
   real F[FV ? FV * FS : 4];
   alignas(16) real sens[AV ? T / 32 * sensor_scratch(P) : 4];
   unsigned long long mx[GRAD ? 1 : 4][GRAD ? 1 : T / 32];   // per-warp max |QDot| as bits (NaN above all)
@@ -357,7 +351,7 @@ __device__ __forceinline__ void node_gradient(const Tl& s, const real* gp, int o
 
 // The traces at both ends of every line of tile U (4 variables) into rec[x * R + v] in global memory (x the
 // element's side node), the variable fastest over the lanes.
-template <int P, int R, bool REL, typename Tl, typename real>
+template <int P, int R, typename Tl, typename real>
 __device__ __forceinline__ void tile_traces(const real* U, const real* c0, const real* c1, real* rec, int n_act, int tid) {
   constexpr int VS = Tl::VS, PO = Tl::PO, FT = Tl::FT;
   for (int x = tid; x < n_act * FT; x += Tl::T) {   // x = (element, line, variable)
@@ -365,11 +359,11 @@ __device__ __forceinline__ void tile_traces(const real* U, const real* c0, const
     real* r = rec + size_t(le) * FT * R + v;
     real in[P];
     load_line<P>(U + v * VS + (le * P + m) * PO, 1, in);
-    r[(3 * P + m) * R] = REL ? trace_dot<P>(c0, in) : dot<P>(c0, in);
-    r[(P + m) * R] = REL ? trace_dot<P>(c1, in) : dot<P>(c1, in);
+    r[(3 * P + m) * R] = dot<P>(c0, in);
+    r[(P + m) * R] = dot<P>(c1, in);
     load_line<P>(U + v * VS + le * P * PO + m, PO, in);
-    r[m * R] = REL ? trace_dot<P>(c0, in) : dot<P>(c0, in);
-    r[(2 * P + m) * R] = REL ? trace_dot<P>(c1, in) : dot<P>(c1, in);
+    r[m * R] = dot<P>(c0, in);
+    r[(2 * P + m) * R] = dot<P>(c1, in);
   }
 }
 
@@ -418,7 +412,7 @@ __device__ __forceinline__ void gradient_traces(Tl& s, const NSOps<P, real>& op,
       }
     }
   } else {
-    if (T_out) tile_traces<P, 4, false, Tl>(s.Q, op.lb0, op.lb1, T_out, n_act, tid);
+    if (T_out) tile_traces<P, 4, Tl>(s.Q, op.lb0, op.lb1, T_out, n_act, tid);
     tile_derivatives<P>(s, op.D, n_act, tid);
     __syncthreads();
     for (int m = tid; m < n_act * NP; m += Tl::T) {
@@ -429,8 +423,8 @@ __device__ __forceinline__ void gradient_traces(Tl& s, const NSOps<P, real>& op,
       for (int k = 0; k < 4; ++k) { s.Fc[k * VS + o] = gx[k]; s.Gc[k * VS + o] = gy[k]; }
     }
     __syncthreads();
-    tile_traces<P, 8, false, Tl>(s.Fc, op.lb0, op.lb1, GT, n_act, tid);
-    tile_traces<P, 8, false, Tl>(s.Gc, op.lb0, op.lb1, GT + 4, n_act, tid);
+    tile_traces<P, 8, Tl>(s.Fc, op.lb0, op.lb1, GT, n_act, tid);
+    tile_traces<P, 8, Tl>(s.Gc, op.lb0, op.lb1, GT + 4, n_act, tid);
   }
 }
 
@@ -524,6 +518,40 @@ __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSAr
   }
 }
 
+// BR1 in float: the volume terms of a node's gradient (hatD along both lines, times the metrics), x and y components.
+template <int P, typename Tl, bool AFFINE, typename real>
+__device__ __forceinline__ void node_volume_gradient(const Tl& s, const real* vg, int le, int node, real* vx, real* vy) {
+  constexpr int VS = Tl::VS, PO = Tl::PO;
+  const int i = node % P, j = node / P;
+  const real *row = &s.Q[(le * P + j) * PO], *col = &s.Q[le * P * PO + i];
+  real ax[4] = {real(0), real(0), real(0), real(0)}, ay[4] = {real(0), real(0), real(0), real(0)};
+#pragma unroll
+  for (int l = 0; l < P; ++l) {
+    const real hi = s.sum.hatT[l * P + i], hj = s.sum.hatT[l * P + j];
+    if constexpr (AFFINE) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        ax[k] += hi * row[k * VS + l];
+        ay[k] += hj * col[k * VS + l * PO];
+      }
+    } else {
+      const real *gx = vg + (j * P + l) * 5, *gy = vg + (l * P + i) * 5;
+      const real j0 = gx[0], j1 = gy[1], j2 = gx[2], j3 = gy[3];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const real qx = row[k * VS + l] * hi, qy = col[k * VS + l * PO] * hj;
+        ax[k] += qx * j0 + qy * j1;
+        ay[k] += qx * j2 + qy * j3;
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    vx[k] = AFFINE ? ax[k] * vg[0] + ay[k] * vg[1] : ax[k];
+    vy[k] = AFFINE ? ax[k] * vg[2] + ay[k] * vg[3] : ay[k];
+  }
+}
+
 // Gradient kernel.  BR1: lifted gradient (stored) and its traces; interior penalty: gradient traces of the
 // resident state.  Then the modal or learned indicator, on the first stage of a time step (and for a bare
 // time derivative); the later stages of the step keep that viscosity.
@@ -542,6 +570,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
   ph.load(a.pc);
   const bool sense = AV && a.sensor.kind != SENSOR_JUMPS && a.first;
   if (sense && a.sensor.kind == SENSOR_LEARNED) sensor_weights_async(s_w, a.sensor.mlp, tid, T);
+  s.sum.fill(op, tid, T);
   pipe.start();
   FlatG flat_g;
   int b = 0, slot = 0;
@@ -551,24 +580,12 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
     typename Tl::In& in = s.in[b];
     const int4* side = s.side[slot];
     const double* Qg = s.state(b);
-    // In float the BR1 gradient is formed from the state minus the element's first node (exactly representable,
-    // subtracted in double): the lifted gradient of a constant vanishes, and the 24-bit rounding of the
-    // state itself and of its contraction -- the largest error of a float time derivative otherwise -- is
-    // taken of the variation instead.  (Not where the indicator reads the tile afterwards, nor in elements
-    // with a mortar side, whose terms hold the whole state.)
-    const auto shift = [&](int le) {
-      bool on = sizeof(real) == 4 && !IP && !sense;
-      if (on && a.NFG)
-        for (int k = 0; k < 4; ++k) on = on && (side[le * 4 + k].y & 15) != SIDE_FLUX;
-      return on;
-    };
     for (int m = tid; m < n_act * NP; m += T) {
       const int o = (m / P) * PO + m % P;
       double q[4];
       ld4(Qg + m * 4, q);
-      const bool sh = shift(m / NP);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) s.Q[k * VS + o] = real(sh ? q[k] - double(real(Qg[(m / NP) * NP * 4 + k])) : q[k]);
+      for (int k = 0; k < 4; ++k) s.Q[k * VS + o] = real(q[k]);
     }
     if constexpr (IP) {
       __syncthreads();
@@ -588,22 +605,18 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
           for (int k = 0; k < 8; ++k) s.F[k * FS + y] = s.one.GTn[x * RG + k];
           continue;
         }
-        real qo[4], us[4], c[4];
+        real qo[4], us[4];
         ld4(&s.one.To[x * RT], qo);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) c[k] = shift(le) ? real(Qg[le * NP * 4 + k]) : real(0);
         const real* g3 = AFFINE ? &in.vg[le * GS + 8 + sd_ * 3] : &s.one.sg[x * 3];
         const real nx = g3[0], ny = g3[1], dS = g3[2];
         if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
           real tp[4];
           ld4(&s.one.Tn[x * RT], tp);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) us[k] = real(0.5) * ((tp[k] - c[k]) + (qo[k] - c[k]));
+          for (int k = 0; k < 4; ++k) us[k] = real(0.5) * (tp[k] + qo[k]);
         } else {
           real uB[4];
           bc_states(ph, a.zones[sd.z], qo, nx, ny, uB, us, sd.w >= 0 ? a.bq + (size_t(sd.w) * P + kk) * 4 : nullptr);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) us[k] -= c[k];
         }
         const real sg = kind == SIDE_RIGHT ? -dS : dS;
 #pragma unroll
@@ -616,8 +629,8 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
       pipe.prefetch(g, b, next_slot);
       pipe.prefetch_rows(g, b, next_slot);
       // per line: minus the volume term plus the lift at its ends, for the x and y components; rows into Fc, Gc,
-      // columns into X, Y
-      for (int x = tid; x < 2 * NF; x += T) {   // x = (direction, variable, element, line)
+      // columns into X, Y.  (Float: the sums of a node in one order, below.)
+      if constexpr (!Tl::SUMS) for (int x = tid; x < 2 * NF; x += T) {   // x = (direction, variable, element, line)
         const int y = x % NF, v = y / (P * EPB), le = (y / P) % EPB, m = y % P;
         if (le >= n_act) continue;
         const bool xi = x < NF;
@@ -651,14 +664,34 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
           dy[o + i * st] = f0[4 * FS] * op.lbw0[i] + f1[4 * FS] * op.lbw1[i] - oy[i];
         }
       }
-      __syncthreads();
+      if constexpr (!Tl::SUMS) __syncthreads();
       for (int m = tid; m < n_act * NP; m += T) {
         const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;
-        const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
         real* gq = a.dQ + size_t(e0 + le) * 8 * NP + node;
+        real iJ, vx[4], vy[4];
+        if constexpr (Tl::SUMS) {
+          iJ = AFFINE ? in.vg[le * GS + 4] : real(1) / a.jac[size_t(e0) * NP + m];
+          node_volume_gradient<P, Tl, AFFINE>(s, &in.vg[le * GS], le, node, vx, vy);
+        } else {
+          iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
+        }
+        const int i = node % P, j = node / P;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const real gx = (s.Fc[k * VS + o] + s.X[k * VS + o]) * iJ, gy = (s.Gc[k * VS + o] + s.Y[k * VS + o]) * iJ;
+          real gx, gy;
+          if constexpr (Tl::SUMS) {
+            const real* f = &s.F[k * FS + le * 4 * PO];   // (side, node): f[side * PO + node], the y components 4 FS on
+            const real lx = f[i] * s.sum.lbw0[j] + f[PO + j] * s.sum.lbw1[i] + f[2 * PO + i] * s.sum.lbw1[j] +
+                            f[3 * PO + j] * s.sum.lbw0[i];
+            const real* h = f + 4 * FS;
+            const real ly = h[i] * s.sum.lbw0[j] + h[PO + j] * s.sum.lbw1[i] + h[2 * PO + i] * s.sum.lbw1[j] +
+                            h[3 * PO + j] * s.sum.lbw0[i];
+            gx = (-vx[k] + lx) * iJ;
+            gy = (-vy[k] + ly) * iJ;
+          } else {
+            gx = (s.Fc[k * VS + o] + s.X[k * VS + o]) * iJ;
+            gy = (s.Gc[k * VS + o] + s.Y[k * VS + o]) * iJ;
+          }
           gq[k * NP] = gx;   // the lifted gradient is not local: stored for the stage kernel
           gq[(4 + k) * NP] = gy;
           s.Fc[k * VS + o] = gx;
@@ -667,8 +700,8 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
       }
       if (a.viscous) {   // gradient traces only feed viscous face fluxes
         __syncthreads();
-        tile_traces<P, 8, false, Tl>(s.Fc, op.lb0, op.lb1, a.GT + size_t(e0) * FT * 8, n_act, tid);
-        tile_traces<P, 8, false, Tl>(s.Gc, op.lb0, op.lb1, a.GT + size_t(e0) * FT * 8 + 4, n_act, tid);
+        tile_traces<P, 8, Tl>(s.Fc, op.lb0, op.lb1, a.GT + size_t(e0) * FT * 8, n_act, tid);
+        tile_traces<P, 8, Tl>(s.Gc, op.lb0, op.lb1, a.GT + size_t(e0) * FT * 8 + 4, n_act, tid);
       }
     }
     if (sense) {
@@ -691,7 +724,7 @@ __device__ __forceinline__ void ns_volume_flux(const Phys<real>& ph, const real*
                                                const real* ax, const real* ay, real mu_v, real mu_l, const real* gp,
                                                real* Fc, real* Gc) {
   real fi[4], gi[4], fv[4], gv[4];
-  inviscid_flux(ph, q, fi, gi);
+  volume_flux(ph, q, fi, gi);
   if (VISC) viscous_flux(ph, q, gx, gy, fv, gv);
   const real Ja00 = gp[0], Ja01 = gp[1], Ja10 = gp[2], Ja11 = gp[3];
 #pragma unroll
@@ -766,7 +799,7 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
   const real lap = (AV && a.av == 1) ? mu_ed * real(one.area[le * 4 + sd_]) : real(0);
   real penalty = real(0);
   if (IP && VISC) penalty = real(a.sigma0) * mu_f * real(P - 1) * real(P - 1) * real(one.invh[le * 4 + sd_]);
-  real F[4];
+  real F[4], fv[4] = {real(0), real(0), real(0), real(0)};   // fv: viscous flux (times dS on a boundary)
   if (kind == SIDE_LEFT || kind == SIDE_RIGHT) {
     const bool right = kind == SIDE_RIGHT;
     real qn[4], QL[4], QR[4];
@@ -783,9 +816,17 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
       ld4(&one.GTn[x * RG + 4], gny);
       viscous_flux(ph, qo, gox, goy, ox, oy);
       viscous_flux(ph, qn, gnx, gny, bx, by);
-      const real hm = real(0.5) * mu_f;
+      if constexpr (IP) {
+        const real hm = real(0.5) * mu_f;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) F[k] -= hm * (ox[k] + bx[k]) * nx + hm * (oy[k] + by[k]) * ny;
+        for (int k = 0; k < 4; ++k) F[k] -= hm * (ox[k] + bx[k]) * nx + hm * (oy[k] + by[k]) * ny;
+      } else {   // LEFT's term first
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const real lx = right ? bx[k] : ox[k], rx = right ? ox[k] : bx[k], ly = right ? by[k] : oy[k], ry = right ? oy[k] : by[k];
+          fv[k] = real(0.5) * (mu_f * lx + mu_f * rx) * nx + real(0.5) * (mu_f * ly + mu_f * ry) * ny;
+        }
+      }
       if (gf) {
         real fgx[4], fgy[4], Ax[4], Ay[4];
 #pragma unroll
@@ -797,11 +838,24 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
         grad_terms(Ax, Ay);
       }
     }
-    const real jump = AV ? penalty + lap : penalty;
+    if constexpr (IP) {
+      const real jump = AV ? penalty + lap : penalty;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if ((IP && VISC) || AV) F[k] += jump * (QL[k] - QR[k]);
-      F[k] *= sg;
+      for (int k = 0; k < 4; ++k) {
+        if (VISC || AV) F[k] += jump * (QL[k] - QR[k]);
+        F[k] *= sg;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (AV) {
+          const real fa = -(lap * (QL[k] - QR[k]));
+          F[k] = (F[k] - fv[k] - fa) * dS;
+        } else {
+          F[k] = (F[k] - fv[k]) * dS;
+        }
+        if (right) F[k] = -F[k];
+      }
     }
   } else {
     const Zone& z = a.zones[sd.z];
@@ -823,9 +877,9 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
         else viscous_flux(ph, qo, gox, goy, Fx, Fy);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          real fv = (mu_f * Fx[k]) * nx + (mu_f * Fy[k]) * ny;
-          if (IP) fv = fv - penalty * (qo[k] - uSB[k]);
-          F[k] -= fv * dS;
+          fv[k] = (mu_f * Fx[k]) * nx + (mu_f * Fy[k]) * ny;
+          if (IP) fv[k] = fv[k] - penalty * (qo[k] - uSB[k]);
+          fv[k] = fv[k] * dS;
         }
         if (gf) {
           real fgx[4], fgy[4];
@@ -840,9 +894,8 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
       }
       if (gf) grad_terms(Gx, Gy);
     }
-    if (AV)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) F[k] += lap * (qo[k] - uSB[k]) * dS;
+    for (int k = 0; k < 4; ++k) F[k] = AV ? F[k] - fv[k] - (-(lap * (qo[k] - uSB[k]))) * dS : F[k] - fv[k];
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) Fo[k * FS] = F[k];
@@ -855,7 +908,8 @@ __device__ __forceinline__ void ns_face_task(const NSArgs<real>& a, const Phys<r
 //   B  (with that gradient) lines: D along both directions; and the gradient-face terms, contracted with hatD along
 //      their side (they enter the lift at every node of a normal line with the same value);
 //   C  (with that gradient) nodes: fluxes;
-//   D  lines: contraction with hatD, lift of the face fluxes (lbw) and the gradient-face terms (lbw, dlbw);
+//   D  lines: contraction with hatD, lift of the face fluxes (lbw) and the gradient-face terms (lbw, dlbw); BR1 in float:
+//      rows of nodes, both directions in one sum (row_sums, hg_stage.cuh);
 //   E  nodes: 1/J, RK update, health check;
 //   F  lines: traces of the new state and, on the fused path, of its gradient; then its indicator.
 template <int P, int V, typename real, bool AFFINE, bool IP, bool AV, bool VISC>
@@ -875,6 +929,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
   const bool gf = IP && VISC && a.grad_faces, rk = a.update && !a.first;
   if (sense && a.sensor.kind == SENSOR_LEARNED) sensor_weights_async(s_w, a.sensor.mlp, tid, T);
   if ((tid & 31) < 4) s.mx[tid & 31][tid >> 5] = 0ull;
+  s.sum.fill(op, tid, T);
   pipe.start();
   FlatG flat_g;
   int b = 0, slot = 0;
@@ -958,7 +1013,16 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
     pipe.prefetch(g, b, next_slot);
 
     // D
-    for (int x = tid; x < 2 * NF; x += T) {   // x = (direction, variable, element, line)
+    if constexpr (Tl::SUMS) {
+      for (int x = tid; x < NF; x += T) {   // x = (variable, element, row)
+        const int v = x / (P * EPB), le = (x / P) % EPB, m = x % P;
+        if (le >= n_act) continue;
+        const real* Fv = &s.F[v * FS + le * 4 * PO];
+        real r[P], *Fc = &s.Fc[v * VS + (le * P + m) * PO];
+        row_sums<P, PO, false>(op, s.sum, Fc, &s.Gc[v * VS + le * P * PO], m, [&](int sd, int k) { return Fv[sd * PO + k]; }, r);
+        store_line<P>(Fc, 1, r);
+      }
+    } else for (int x = tid; x < 2 * NF; x += T) {   // x = (direction, variable, element, line)
       const int y = x % NF, v = y / (P * EPB), le = (y / P) % EPB, m = y % P;
       if (le >= n_act) continue;
       const bool xi = x < NF;
@@ -1003,7 +1067,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
       if (on) {
         const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) qd[k] = (s.Fc[k * VS + o] + s.Gc[k * VS + o]) * iJ;
+        for (int k = 0; k < 4; ++k) qd[k] = (Tl::SUMS ? s.Fc[k * VS + o] : s.Fc[k * VS + o] + s.Gc[k * VS + o]) * iJ;
       }
       if (a.resid)   // the whole warp takes part
 #pragma unroll
@@ -1050,7 +1114,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
       if (IP && VISC && a.fuse)   // the side tile is free since the lift
         gradient_traces<P, AFFINE>(s, op, in.vg, T_out, a.GT_out + size_t(e0) * FT * 8, n_act, tid);
       else
-        tile_traces<P, 4, !IP, Tl>(s.Q, op.lb0, op.lb1, T_out, n_act, tid);
+        tile_traces<P, 4, Tl>(s.Q, op.lb0, op.lb1, T_out, n_act, tid);
       if constexpr (IP && AV) {
         if (sense) {
           __syncthreads();

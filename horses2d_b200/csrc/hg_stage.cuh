@@ -13,7 +13,7 @@
 //      fluxes (Scalar_StdVolumeGreen, Approximation/DGWeakIntegrals.f90:111-181);
 //   B  one thread per (variable, line of nodes, direction): the line's P fluxes in registers, contracted
 //      with hatD and lifted with lbw at its two ends (Scalar_StdFace, DGWeakIntegrals.f90:183-266), back
-//      in place;
+//      in place; in float one thread per (variable, row of nodes) for both directions (row_sums);
 //   C  per node: division by J (computeQDot :226-233), low-storage RK update G = a G + b QDot,
 //      Q += c G (DGTimeIntegrator.f90:282-365); Gauss-Lobatto: the boundary nodes are the new traces;
 //   D  Legendre-Gauss: one thread per (variable, line): the traces of the new state at the line's ends
@@ -237,6 +237,48 @@ __device__ __forceinline__ void check_state(int* health, int* health_host, doubl
 __host__ __device__ constexpr int face_node(int P, int side, int l, int kk) {
   return (side == 0 || side == 2) ? (l * P + kk) : (kk * P + l);
 }
+
+// In float a node's contraction and lift are one sum in one order: for l = 0 .. N the xi term, then the eta term,
+// then the bottom, right, top and left sides.  A 32-bit time derivative of a smooth state is a difference of sums a
+// thousand times as large, so another order gives it other digits from the fourth on (the two directions summed
+// apart: 3e-4 in the 2-norm at N = 8, against 5e-11 in double, whose kernels do that: one line of one direction per
+// thread).  The lanes of a row of nodes hold different rows j of hatD: a copy in shared memory, transposed.
+template <int P, typename real, bool USED = sizeof(real) == 4>
+struct SumOps {
+  static constexpr bool ON = USED;
+  real hatT[ON ? P * P : 1], lbw0[ON ? P : 1], lbw1[ON ? P : 1];
+  template <typename Ops>
+  __device__ __forceinline__ void fill(const Ops& op, int tid, int T) {
+    if constexpr (ON) {
+      for (int k = tid; k < P * P; k += T) hatT[(k % P) * P + k / P] = op.hatD[k];
+      for (int k = tid; k < P; k += T) { lbw0[k] = op.lbw0[k]; lbw1[k] = op.lbw1[k]; }
+    }
+  }
+};
+// The sums of row j of an element, of one variable: Fc the row of xi fluxes, Gc the element's tile of eta fluxes (rows of
+// PO nodes); face(side, k) the side's flux at its node k.  out replaces the row of xi fluxes.
+template <int P, int PO, bool ENDS, typename Ops, typename real, typename Face>
+__device__ __forceinline__ void row_sums(const Ops& op, const SumOps<P, real, true>& so, const real* Fc, const real* Gc, int j,
+                                         Face face, real (&out)[P]) {
+  real f[P], hj[P];
+#pragma unroll
+  for (int l = 0; l < P; ++l) {
+    f[l] = Fc[l];
+    hj[l] = so.hatT[l * P + j];
+  }
+  const real b0 = so.lbw0[j], b1 = so.lbw1[j], Fr = face(1, j), Fl = face(3, j);
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    real r = real(0);
+#pragma unroll
+    for (int l = 0; l < P; ++l) r = r + op.hatD[i * P + l] * f[l] + hj[l] * Gc[l * PO + i];
+    if (!ENDS || j == 0) r = r - face(0, i) * b0;
+    if (!ENDS || i == P - 1) r = r - Fr * op.lbw1[i];
+    if (!ENDS || j == P - 1) r = r - face(2, i) * b1;
+    if (!ENDS || i == 0) r = r - Fl * op.lbw0[i];
+    out[i] = r;
+  }
+}
 // Shared memory of a stage CTA.
 template <int P, int V, typename real, bool AFFINE, bool LGL>
 struct StageTiles {
@@ -256,6 +298,7 @@ struct StageTiles {
   alignas(16) int4 side[3][EPB * 4];
   real Fc[4 * VS], Gc[4 * VS];      // contravariant fluxes, then their contractions; Fc then holds the new state
   real F[4 * NF];                   // face fluxes x dS (signed for a RIGHT side)
+  SumOps<P, real> sum;
   uint64_t bar[2];
 };
 
@@ -269,6 +312,7 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     stage_kernel(const __grid_constant__ StageArgs<real> a, const __grid_constant__ StageOps<P, real> op) {
   using Tl = StageTiles<P, V, real, AFFINE, LGL>;
   constexpr int EPB = Tl::EPB, T = Tl::T, NP = Tl::NP, FT = Tl::FT, PO = Tl::PO, NF = Tl::NF, VS = Tl::VS, GS = Tl::GS;
+  constexpr bool SUMS = SumOps<P, real>::ON;
   extern __shared__ __align__(16) unsigned char stage_smem[];
   Tl& s = *reinterpret_cast<Tl*>(stage_smem);
   const int tid = threadIdx.x;
@@ -314,6 +358,7 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     cp_async_commit();
   };
 
+  s.sum.fill(op, tid, T);
   if (tid == 0) {
     mbar_init(&s.bar[0]);
     mbar_init(&s.bar[1]);
@@ -408,7 +453,7 @@ __global__ void __launch_bounds__(stage_threads(P, V))
         const real* gp = AFFINE ? &in.vg[le * GS] : &in.vg[le * GS + node * 5];
         const real Ja00 = gp[0], Ja01 = gp[1], Ja10 = gp[2], Ja11 = gp[3];
         real f[4], gg[4];
-        inviscid_flux(ph, q, f, gg);
+        volume_flux(ph, q, f, gg);
         const int o = (le * P + node / P) * PO + node % P;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -441,14 +486,23 @@ __global__ void __launch_bounds__(stage_threads(P, V))
       const int v = x / (P * EPB), le = (x / P) % EPB, m = x % P;
       if (le >= n_act) continue;
       const real* Fv = &s.F[v * NF + le * FT];
-      line(&s.Fc[v * VS + (le * P + m) * PO], 1, Fv[3 * P + m], Fv[P + m]);
+      real* Fc = &s.Fc[v * VS + (le * P + m) * PO];
+      if constexpr (SUMS) {
+        real r[P];
+        row_sums<P, PO, LGL>(op, s.sum, Fc, &s.Gc[v * VS + le * P * PO], m, [&](int sd, int k) { return Fv[sd * P + k]; }, r);
+#pragma unroll
+        for (int l = 0; l < P; ++l) Fc[l] = r[l];
+      } else {
+        line(Fc, 1, Fv[3 * P + m], Fv[P + m]);
+      }
     }
-    for (int x = tid; x < NF; x += T) {
-      const int v = x / (P * EPB), le = (x / P) % EPB, m = x % P;
-      if (le >= n_act) continue;
-      const real* Fv = &s.F[v * NF + le * FT];
-      line(&s.Gc[v * VS + le * P * PO + m], PO, Fv[m], Fv[2 * P + m]);
-    }
+    if constexpr (!SUMS)
+      for (int x = tid; x < NF; x += T) {
+        const int v = x / (P * EPB), le = (x / P) % EPB, m = x % P;
+        if (le >= n_act) continue;
+        const real* Fv = &s.F[v * NF + le * FT];
+        line(&s.Gc[v * VS + le * P * PO + m], PO, Fv[m], Fv[2 * P + m]);
+      }
     __syncthreads();
 
     // C: time derivative and update, W variables of a node to a lane.  In double two lanes share a node: 16-byte
@@ -464,7 +518,8 @@ __global__ void __launch_bounds__(stage_threads(P, V))
       if (on) {
         const real iJ = AFFINE ? in.vg[le * GS + 4] : in.vg[le * GS + node * 5 + 4];
 #pragma unroll
-        for (int k = 0; k < W; ++k) qd[k] = (s.Fc[(h + k) * VS + o] + s.Gc[(h + k) * VS + o]) * iJ;
+        for (int k = 0; k < W; ++k)
+          qd[k] = (SUMS ? s.Fc[(h + k) * VS + o] : s.Fc[(h + k) * VS + o] + s.Gc[(h + k) * VS + o]) * iJ;
         if (a.QDot) {
           double dq[W];
 #pragma unroll
@@ -546,12 +601,10 @@ __global__ void __launch_bounds__(stage_threads(P, V))
 
 // Traces of the resident state (after hg_set_state).
 // Summed in the order of the stage kernels, so that a state loaded from the host has the traces bit for bit that
-// a stage left.  how = TRACE_NODAL: the Euler kernel's Gauss-Lobatto traces, the end nodes themselves;
-// TRACE_RELATIVE: BR1's, in float relative to the line's first node.
-enum { TRACE_PLAIN = 0, TRACE_NODAL = 1, TRACE_RELATIVE = 2 };
+// a stage left.  nodal: the Euler kernel's Gauss-Lobatto traces, the end nodes themselves.
 template <int P, int EPB, typename real>
 __global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const double* Q, const double* mats, real* T,
-                                                             int how) {
+                                                             bool nodal) {
   constexpr int NP = P * P;
   constexpr int FT = 4 * P;
   __shared__ real s_lb[2 * P];
@@ -570,20 +623,13 @@ __global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const dou
     const int s = t / P, kk = t % P;
     const real* lbv = (s == 0 || s == 3) ? s_lb : s_lb + P;
     real tr[4] = {real(0), real(0), real(0), real(0)};
-    if (how == TRACE_NODAL) {
+    if (nodal) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) tr[k] = s_Q[k][le][face_node(P, s, (s == 0 || s == 3) ? 0 : P - 1, kk)];
-    } else if (sizeof(real) == 8 || how == TRACE_PLAIN) {
+    } else {
       for (int l = 0; l < P; ++l)
 #pragma unroll
         for (int k = 0; k < 4; ++k) tr[k] += s_Q[k][le][face_node(P, s, l, kk)] * lbv[l];
-    } else {
-      const int n0 = face_node(P, s, 0, kk);
-      for (int l = 1; l < P; ++l)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tr[k] += (s_Q[k][le][face_node(P, s, l, kk)] - s_Q[k][le][n0]) * lbv[l];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) tr[k] = s_Q[k][le][n0] + tr[k];
     }
     real* tp = T + ((size_t(e) * 4 + s) * P + kk) * 4;
 #pragma unroll
