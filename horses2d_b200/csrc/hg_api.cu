@@ -643,7 +643,7 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
   c->d_T[0] = dalloc<char>(size_t(E) * 4 * P * 4 * rs);
   c->d_T[1] = dalloc<char>(size_t(E) * 4 * P * 4 * rs);
   c->d_QDot = dalloc<double>(c->ndof);
-  c->d_resid = dalloc<double>(size_t(max_grid(c)) * 4);
+  c->d_resid = dalloc<double>((size_t(max_grid(c)) + 1) * 4);
   c->d_resid_out = dalloc<double>(4);
   c->d_elmax = dalloc<double>(size_t(E) * 4);
   if (c->av != HG_AV_NONE) {
@@ -720,7 +720,7 @@ void ctx_build(hg_ctx* c, const hg_mesh_desc* m, const hg_physics_desc* ph, cons
   c->h_mats = mats;
   HG_CUDA(cudaMemcpy(c->d_mats, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
   HG_CUDA(cudaMemcpy(c->d_zones, zones.data(), zones.size() * sizeof(Zone), cudaMemcpyHostToDevice));
-  HG_CUDA(cudaMemset(c->d_resid, 0, size_t(max_grid(c)) * 4 * sizeof(double)));
+  HG_CUDA(cudaMemset(c->d_resid, 0, (size_t(max_grid(c)) + 1) * 4 * sizeof(double)));
 }
 
 extern "C" int hg_create(const hg_mesh_desc* mesh, const hg_physics_desc* phys, const hg_bc_desc* bcs, int32_t n_bcs,
@@ -1027,7 +1027,7 @@ extern "C" int hg_residuals(hg_ctx* c, double out[4]) {
       return 0;
     }
     timed(c, HG_KERNEL_REDUCE,
-          [&] { residual_reduce_kernel<<<1, 256, 0, c->stream>>>(c->n_resid, c->d_resid, c->d_resid_out); });
+          [&] { residual_reduce_kernel<<<1, 256, 0, c->stream>>>(c->d_resid, c->d_resid_out); });
     ++c->launches;
     HG_CUDA(cudaGetLastError());
     HG_CUDA(cudaMemcpyAsync(out, c->d_resid_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

@@ -33,8 +33,7 @@ struct hg_ctx {
   void* d_G = nullptr;
   void* d_T[2] = {nullptr, nullptr};
   double* d_QDot = nullptr;
-  double* d_resid = nullptr;      // per-CTA partial maxima of |QDot| of the last stage [n_resid][4]
-  int n_resid = 1;                // CTAs of that stage
+  double* d_resid = nullptr;      // per-CTA partial maxima of |QDot| of the last stage (put_partial, hg_stage.cuh)
   double* d_resid_out = nullptr;  // reduced maxima [4]
   double* d_elmax = nullptr;      // [n_el][4] umax, amax per element and their NaN flags
   int cur = 0;                    // which trace buffer holds the current traces

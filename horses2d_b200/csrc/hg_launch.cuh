@@ -67,7 +67,6 @@ static void launch_stage_PAL(hg_ctx* c, const StageArgs<real>& a) {
   const int most = c->n_sm * std::min(32, resident_ctas(c, known, stage_kernel<P, V, real, AFFINE, LGL>, Tl::T, sizeof(Tl), sizeof(Tl)));
   // every CTA takes the same number of groups but the last ones: no more CTAs than that needs
   const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
-  if (a.resid) c->n_resid = grid;
   const StageOps<P, real> op = stage_ops<P, real>(c);
   timed(c, HG_KERNEL_STAGE, [&] { launch_dependent(c, stage_kernel<P, V, real, AFFINE, LGL>, grid, Tl::T, sizeof(Tl), a, op); });
   ++c->launches;
@@ -121,9 +120,9 @@ static NSOps<P, real> ns_ops(const hg_ctx* c) {
   return o;
 }
 
-// Persistent launch of a Navier-Stokes kernel with tiles Tl; returns its CTAs.
+// Persistent launch of a Navier-Stokes kernel with tiles Tl.
 template <typename Tl, typename K, typename A, typename O>
-static int launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind, bool weights, const A& a, const O& op) {
+static void launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind, bool weights, const A& a, const O& op) {
   static_assert(sizeof(Tl) + MLP_BYTES <= 227 * 1024, "shared memory of a CTA");
   const size_t smem = sizeof(Tl) + (weights ? MLP_BYTES : 0);
   const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
@@ -131,7 +130,6 @@ static int launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind,
   const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
   timed(c, kind, [&] { launch_dependent(c, kernel, grid, Tl::T, smem, a, op); });
   ++c->launches;
-  return grid;
 }
 
 template <int P, typename real, int V, bool AFFINE, bool IP, bool AV>
@@ -152,17 +150,15 @@ static void launch_ns_PAI(hg_ctx* c, const NSArgs<real>& a) {
   }
   if (a.run_stage) {
     const bool w = learned && a.fuse && a.update && a.last;
-    int grid;
     if (!AV || a.viscous) {
       using Tl = NSTiles<P, V, real, AFFINE, IP, AV, true, false>;
       static std::atomic<int> known[2][HG_KNOWN_DEVICES];
-      grid = launch_groups<Tl>(c, known[w], ns_stage_kernel<P, V, real, AFFINE, IP, AV, true>, HG_KERNEL_STAGE, w, a, op);
+      launch_groups<Tl>(c, known[w], ns_stage_kernel<P, V, real, AFFINE, IP, AV, true>, HG_KERNEL_STAGE, w, a, op);
     } else {
       using Tl = NSTiles<P, V, real, AFFINE, IP, AV, !AV, false>;
       static std::atomic<int> known[2][HG_KNOWN_DEVICES];
-      grid = launch_groups<Tl>(c, known[w], ns_stage_kernel<P, V, real, AFFINE, IP, AV, !AV>, HG_KERNEL_STAGE, w, a, op);
+      launch_groups<Tl>(c, known[w], ns_stage_kernel<P, V, real, AFFINE, IP, AV, !AV>, HG_KERNEL_STAGE, w, a, op);
     }
-    if (a.resid) c->n_resid = grid;
   }
 }
 

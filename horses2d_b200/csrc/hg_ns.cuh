@@ -1133,7 +1133,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
     if (tid < 4) {
       unsigned long long m = 0ull;
       for (int w = 0; w < T / 32; ++w) m = s.mx[tid][w] > m ? s.mx[tid][w] : m;
-      a.resid[size_t(blockIdx.x) * 4 + tid] = __longlong_as_double((long long)m);
+      put_partial(a.resid, tid, __longlong_as_double((long long)m));
     }
   }
 }

@@ -59,7 +59,7 @@ struct StageArgs {
   const real* T_in;        // [n_el*4][P][4]
   real* T_out;
   double* QDot;            // optional output (time derivative only)
-  double* resid;           // optional per-CTA max |QDot| per variable: [gridDim.x][4]
+  double* resid;           // optional per-CTA max |QDot| per variable (put_partial)
   int* health;             // device health word {bits, element} (check_state), may be null
   int* health_host;        // mapped host flag set beside it, may be null
   double a, b, c;          // G = a G + b QDot ; Q += c G
@@ -191,10 +191,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
 // max that keeps NaN (a residual that is NaN must stay visible)
 __device__ __forceinline__ double nanmax(double m, double v) { return (v > m || v != v) ? v : m; }
 
+// Residual partials of a launch: {CTAs, -, -, -}, then a row of 4 maxima per CTA.  The count stands beside them because
+// launches of one kernel differ in their CTAs (the network's weights take shared memory on the last stage of a step) and
+// a replayed graph passes no host code that could note it.
+__device__ __forceinline__ void put_partial(double* resid, int k, double m) {
+  resid[4 + size_t(blockIdx.x) * 4 + k] = m;
+  if (blockIdx.x == 0 && k == 0) resid[0] = double(gridDim.x);
+}
+
 // Per-CTA residual maxima from each lane's W variables (W = 2: even lanes 0 and 1, odd lanes 2 and 3); scratch holds
 // W T values.
 template <int W, int T>
-__device__ __forceinline__ void residual_partial(const double* mx, double* scratch, double* out, int tid) {
+__device__ __forceinline__ void residual_partial(const double* mx, double* scratch, double* resid, int tid) {
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < W; ++k) scratch[W * tid + k] = mx[k];
@@ -202,7 +210,7 @@ __device__ __forceinline__ void residual_partial(const double* mx, double* scrat
   if (tid < 4) {
     double m = 0.0;
     for (int t = tid; t < W * T; t += 4) m = nanmax(m, scratch[t]);
-    out[tid] = m;
+    put_partial(resid, tid, m);
   }
 }
 
@@ -595,7 +603,7 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     b ^= 1;
     slot = next_slot;
   }
-  if (a.resid) residual_partial<W, T>(mx, reinterpret_cast<double*>(s.in), a.resid + size_t(blockIdx.x) * 4, tid);
+  if (a.resid) residual_partial<W, T>(mx, reinterpret_cast<double*>(s.in), a.resid, tid);
   static_assert(sizeof(s.in) >= W * T * sizeof(double), "scratch of the residual maxima");
 }
 
@@ -637,8 +645,10 @@ __global__ void __launch_bounds__(block_for(P)) trace_kernel(int n_el, const dou
   }
 }
 
-// Max over the per-CTA residual partials: out[k] = max_b part[b*4+k] (NaN kept).
-static __global__ void residual_reduce_kernel(int nblocks, const double* part, double* out) {
+// Max over the per-CTA residual partials (NaN kept).
+static __global__ void residual_reduce_kernel(const double* resid, double* out) {
+  const int nblocks = int(resid[0]);
+  const double* part = resid + 4;
   __shared__ double s[4][256];
   double m[4] = {0.0, 0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
