@@ -20,7 +20,7 @@ BC_PERIODIC, BC_DIRICHLET, BC_EULERWALL, BC_VISCOUSWALL, BC_FARFIELD, BC_PRESSUR
 BC_NEWDIRICHLET = 7
 AV_NONE, AV_LAPLACIAN, AV_PHYSICAL = 0, 1, 2
 STATUS_CRASHED = 2
-HEALTH_NONFINITE, HEALTH_DENSITY, HEALTH_PRESSURE = 1, 2, 4
+HEALTH_NONFINITE, HEALTH_DENSITY, HEALTH_PRESSURE, HEALTH_COPY = 1, 2, 4, 8
 
 I32P = C.POINTER(C.c_int32)
 F64P = C.POINTER(C.c_double)

@@ -246,6 +246,7 @@ static void run_ns_stage(hg_ctx* c, double ca, double cb, double cc, bool first,
   a.sensor = sensor_args(c);
   a.health = c->d_health;
   a.health_host = c->d_health_flag;
+  a.polls = c->copy_polls;
   a.run_stage = c->ns_phase != 1;
   if (c->ns_phase == 2) a.run_gradient = a.run_jumps = 0;
   a.fuse = (ns_fused(c) && !c->prologue) ? 1 : 0;
@@ -283,6 +284,7 @@ static void run_stage(hg_ctx* c, double ca, double cb, double cc, bool first, bo
   a.resid = resid ? c->d_resid : nullptr;
   a.health = c->d_health;
   a.health_host = c->d_health_flag;
+  a.polls = c->copy_polls;
   a.a = ca; a.b = cb; a.c = cc;
   a.first = first ? 1 : 0;
   a.update = update ? 1 : 0;
@@ -879,6 +881,7 @@ extern "C" int hg_time_derivative(hg_ctx* c, double t, double* QDot) {
       HG_CUDA(cudaMemcpyAsync(QDot, c->d_QDot, c->ndof * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
       HG_CUDA(cudaStreamSynchronize(c->stream));
     }
+    if (QDot) health_check(c);
     return 0;
   } catch (const std::exception& ex) { return fail(c, ex); }
 }
@@ -1130,6 +1133,19 @@ extern "C" int hg_health(hg_ctx* c, int32_t* bits, int32_t* element) {
     HG_CUDA(cudaMemcpy(w, c->d_health, sizeof(w), cudaMemcpyDeviceToHost));
     if (bits) *bits = w[0];
     if (element) *element = w[1];
+    return 0;
+  } catch (const std::exception& ex) { return fail(c, ex); }
+}
+
+// For the tests of the failure report, not part of the interface: the poll limit of the stage kernels' waits for their
+// copies; with 0 every wait gives up at once, n < 0 sets the limit back.
+extern "C" int hg_test_copy_polls(hg_ctx* c, int32_t n) {
+  try {
+    if (!c) return 1;
+    HG_CUDA(cudaStreamSynchronize(c->stream));
+    drop_graph(c);
+    c->copy_polls = n < 0 ? COPY_POLLS : n;
+    for (hg_ctx* p : c->parts) p->copy_polls = c->copy_polls;
     return 0;
   } catch (const std::exception& ex) { return fail(c, ex); }
 }

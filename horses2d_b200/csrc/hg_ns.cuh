@@ -81,6 +81,7 @@ struct NSArgs {
   double* mu_next;          //   mu_next
   int* health;              // device health word {bits, first element} (check_state)
   int* health_host;         // mapped host flag set beside it
+  int polls;                // limit of a wait for copies (mbar_wait)
 };
 
 // Elements per group and threads per CTA: variant 0, and variant 1 for small meshes.  At order 5 a double group is
@@ -200,10 +201,6 @@ struct NSPipe {
   unsigned phase = 0u;   // parities of the barriers
 
   __device__ __forceinline__ int count(int g) const { return min(EPB, a.n_el - g * EPB); }
-  __device__ __forceinline__ void gave_up() const {
-    if (a.health) atomicOr(a.health, HEALTH_COPY);
-    if (a.health_host) *reinterpret_cast<volatile int*>(a.health_host) = 1;
-  }
   // inputs of group g (those of struct In into half b), and the side table of the group after it (thread 0)
   // first: of the CTA's first group, where the constant ones (tables, metrics) go ahead of the wait for the kernel before
   __device__ __forceinline__ void bulk(int g, int b, bool first, int slot) const {
@@ -286,22 +283,32 @@ struct NSPipe {
     rows(blockIdx.x, 0, side0, at0);
     __syncthreads();   // the barriers are initialised
   }
-  __device__ __forceinline__ void wait(int k) {
-    if (!mbar_wait(&s.bar[k], (phase >> k) & 1u)) gave_up();
+  // Waits for the copies of barrier k, then for the CTA: false (in every thread) where a thread gave up.
+  __device__ __forceinline__ bool wait(int k) {
+    const bool late = !mbar_wait(&s.bar[k], (phase >> k) & 1u, a.polls);
+    if (k == 0) cp_async_wait_all();
+    if (__syncthreads_or(late)) return false;
     phase ^= 1u << k;
+    return true;
+  }
+  // ... and then: copies of barrier 0 (the inputs of group g or, while g is worked on, of the group after it) and of
+  // barrier 1 may be in flight
+  __device__ __forceinline__ void failed(int g, bool working) const {
+    if (tid != 0) return;
+    if (!working || g + int(gridDim.x) < n_groups) copies_failed(a.health, a.health_host, &s.bar[0], phase & 1u);
+    if (working) copies_failed(a.health, a.health_host, &s.bar[1], (phase >> 1) & 1u);
   }
   // top of the loop for group g: its inputs are there, every thread is done with the group before, and its RK
   // register is on its way
-  __device__ __forceinline__ void next(int g, bool rk) {
-    wait(0);
-    cp_async_wait_all();
-    __syncthreads();
+  __device__ __forceinline__ bool next(int g, bool rk) {
+    if (!wait(0)) { failed(g, false); return false; }
     if (g + int(gridDim.x) >= n_groups) grid_launch_next();   // the CTA's last group
     if (rk && tid == 0) {
       const unsigned bytes = count(g) * NP * 4u * unsigned(sizeof(real));
       mbar_expect(&s.bar[1], bytes);
       bulk_copy(s.G, a.G + size_t(g) * EPB * NP * 4, bytes, &s.bar[1]);
     }
+    return true;
   }
   // after the barrier behind the face tasks: the next group's records
   __device__ __forceinline__ void prefetch_rows(int g, int b, int next_slot) const {
@@ -576,7 +583,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8))
   int b = 0, slot = 0;
   for (int g = blockIdx.x; g < n_groups; g += gridDim.x) {
     const int e0 = g * EPB, n_act = pipe.count(g), next_slot = slot == 2 ? 0 : slot + 1;
-    pipe.next(g, false);
+    if (!pipe.next(g, false)) return;
     typename Tl::In& in = s.in[b];
     const int4* side = s.side[slot];
     const double* Qg = s.state(b);
@@ -935,7 +942,7 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
   int b = 0, slot = 0;
   for (int g = blockIdx.x; g < n_groups; g += gridDim.x) {
     const int e0 = g * EPB, n_act = pipe.count(g), next_slot = slot == 2 ? 0 : slot + 1;
-    pipe.next(g, rk);
+    if (!pipe.next(g, rk)) return;
     typename Tl::In& in = s.in[b];
     const int4* side = s.side[slot];
     bool local = IP && VISC;   // the volume fluxes need the element-local gradient (uniform over the CTA)
@@ -1055,10 +1062,14 @@ __global__ void __launch_bounds__(ns_threads(P, V, sizeof(real) == 8), ns_min_ct
       if (xi) line(&s.Fc[v * VS + (le * P + m) * PO], 1);
       else line(&s.Gc[v * VS + le * P * PO + m], PO);
     }
-    __syncthreads();
+    if (!rk) {
+      __syncthreads();
+    } else if (!pipe.wait(1)) {
+      pipe.failed(g, true);
+      return;
+    }
 
     // E
-    if (rk) pipe.wait(1);
     for (int m = tid; m < (Tl::NN + 31) / 32 * 32; m += T) {
       const bool on = m < n_act * NP;
       const int le = m / NP, node = m % NP, o = (m / P) * PO + node % P;

@@ -62,12 +62,16 @@ struct StageArgs {
   double* resid;           // optional per-CTA max |QDot| per variable (put_partial)
   int* health;             // device health word {bits, element} (check_state), may be null
   int* health_host;        // mapped host flag set beside it, may be null
+  int polls;               // limit of a wait for copies (mbar_wait)
   double a, b, c;          // G = a G + b QDot ; Q += c G
   int first;               // a == 0: do not read G
   int update;              // 1: RK update, 0: only QDot (and traces of the unchanged Q)
   int riemann;
   PhysConst pc;
 };
+
+// Bits of the health word (check_state; COPY: copies_failed).
+enum { HEALTH_NONFINITE = 1, HEALTH_DENSITY = 2, HEALTH_PRESSURE = 4, HEALTH_COPY = 8 };
 
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
@@ -176,16 +180,26 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 __device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 // Waits for the phase; gives up after a bounded number of polls (each suspends the thread for a while) and
-// reports false, so that a copy which never lands ends the launch instead of hanging it.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
+// reports false.  The CTA's threads then leave together (copies_failed), before any of them reads what the copies
+// should have brought: a copy that never lands ends the launch with a health bit instead of hanging it.
+constexpr int COPY_POLLS = 1 << 20;
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int polls) {
   const unsigned b = static_cast<unsigned>(__cvta_generic_to_shared(bar));
-  for (int n = 0; n < (1 << 20); ++n) {
+  for (int n = 0; n < polls; ++n) {
     unsigned done;
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(done) : "r"(b), "r"(parity) : "memory");
     if (done) return true;
   }
   return false;
+}
+
+// Of the CTA's threads that gave up waiting (any: uniform): the health bit, and a last bounded wait for the copies
+// still in flight, which must not outlive the CTA's shared memory.
+__device__ __forceinline__ void copies_failed(int* health, int* health_host, uint64_t* bar, unsigned parity) {
+  if (health) atomicOr(health, HEALTH_COPY);
+  if (health_host) *reinterpret_cast<volatile int*>(health_host) = 1;
+  mbar_wait(bar, parity, COPY_POLLS);
 }
 
 // max that keeps NaN (a residual that is NaN must stay visible)
@@ -228,7 +242,6 @@ __device__ __forceinline__ unsigned long long warp_max_bits(double v) {
 // bit 2 rho <= 0, bit 4 p <= 0 (tested as rho (rho E) - |rho u|^2 / 2 = rho p / (gamma - 1) <= 0, no
 // division).  health = {bits, an offending element (the first to arrive)}; the mapped host flag tells
 // the host without a synchronisation that the word is no longer clean.
-enum { HEALTH_NONFINITE = 1, HEALTH_DENSITY = 2, HEALTH_PRESSURE = 4, HEALTH_COPY = 8 };   // COPY: mbar_wait gave up
 __device__ __forceinline__ void check_state(int* health, int* health_host, double r, double ru, double rv,
                                             double rE, int e) {
   const bool finite = fabs(r) + fabs(ru) + fabs(rv) + fabs(rE) < 1.0e300;
@@ -385,13 +398,14 @@ __global__ void __launch_bounds__(stage_threads(P, V))
   unsigned phase = 0u;
   for (int g = blockIdx.x; g < n_groups; g += gridDim.x) {
     const int e0 = g * EPB, n_act = count(g);
-    if (!mbar_wait(&s.bar[b], (phase >> b) & 1u) && tid == 0) {
-      if (a.health) atomicOr(a.health, HEALTH_COPY);
-      if (a.health_host) *reinterpret_cast<volatile int*>(a.health_host) = 1;
+    const bool late = !mbar_wait(&s.bar[b], (phase >> b) & 1u, a.polls);
+    cp_async_wait_all();
+    // (the barrier: every thread is done with the previous group, its half and the work tiles are free)
+    if (__syncthreads_or(late)) {
+      if (tid == 0) copies_failed(a.health, a.health_host, &s.bar[b], (phase >> b) & 1u);
+      return;
     }
     phase ^= 1u << b;
-    cp_async_wait_all();
-    __syncthreads();   // every thread is done with the previous group: its half and the work tiles are free
     const int next_slot = slot == 2 ? 0 : slot + 1;
     if (g + int(gridDim.x) < n_groups) {
       if (tid == 0) issue_bulk(g + gridDim.x, b ^ 1, false, next_slot);

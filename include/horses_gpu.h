@@ -148,9 +148,11 @@ int  hg_residuals(hg_ctx* ctx, double out[4]);
  * of each step call (so the call after the bad step reports it), and at once by the synchronising
  * calls (hg_residuals, hg_get_state, hg_estimate_dt, hg_synchronize).  The record stays until
  * hg_set_state replaces the state.  hg_health synchronises and returns the bits (0: clean) and the
- * element (-1 when clean). */
+ * element (-1 when clean).
+ * HG_HEALTH_COPY is not a property of the state: a stage kernel gave up waiting for its own copies and left part of the
+ * elements as they were.  It fails the same calls, and hg_time_derivative, with status 1 whatever the policy. */
 enum { HG_STATUS_CRASHED = 2 };
-enum { HG_HEALTH_NONFINITE = 1, HG_HEALTH_DENSITY = 2, HG_HEALTH_PRESSURE = 4 };
+enum { HG_HEALTH_NONFINITE = 1, HG_HEALTH_DENSITY = 2, HG_HEALTH_PRESSURE = 4, HG_HEALTH_COPY = 8 };
 int  hg_health(hg_ctx* ctx, int32_t* bits, int32_t* element);
 int  hg_set_health_policy(hg_ctx* ctx, int32_t fatal_bits);
 /* == EstimateTimeStep, including the reference's running maxima (SAVE). */
