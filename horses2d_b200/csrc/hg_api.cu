@@ -119,19 +119,17 @@ static void health_check(hg_ctx* c) {
                 "); set a new state to continue");
 }
 
-// Tiling of the stage kernels: variant 0's groups of elements are cut to variant 1's where they would
-// leave half of the SMs or more without one (fewer than two groups per SM): there a stage is one pass of
-// latency, and the smaller groups spread it over the chip.
-// (Navier-Stokes orders 9 and 10 run one element per group in both variants, one instantiation.)
+// Tiling of the stage kernels.  Until a variant is set (hg_set_tiling, hg_autotune), variant 1 where variant 0's groups
+// of elements would leave half of the SMs or more without one (fewer than two groups per SM): there a stage is one pass
+// of latency, and the smaller groups spread it over the chip (an RK3 step at N = 4 in double: 800 elements 15.9 us with
+// variant 0 and 12.8 with variant 1, 16,000 elements 77 and 107).
 static bool in_double(const hg_ctx* c) { return c->precision == HG_PREC_FP64; }
-static int stage_variant(const hg_ctx* c, int variant) {
-  if (c->ns && c->P >= 10) return 0;
-  return variant || c->n_el < 2 * c->n_sm * (c->ns ? epb_ns_of(c->P, 0, in_double(c)) : epb_stage(c->P, 0)) ? 1 : 0;
+static int tiling_of(const hg_ctx* c) {
+  if (c->tiling >= 0) return c->tiling;
+  return c->n_el < 2 * c->n_sm * (c->ns ? epb_ns_of(c->P, 0, in_double(c)) : epb_stage(c->P, 0)) ? 1 : 0;
 }
-static int epb_of(const hg_ctx* c, int variant) {
-  const int v = stage_variant(c, variant);
-  return c->ns ? epb_ns_of(c->P, v, in_double(c)) : epb_stage(c->P, v);
-}
+// The kernels' variant: Navier-Stokes orders 9 and 10 run one element per group in both, one instantiation.
+static int stage_variant(const hg_ctx* c) { return c->ns && c->P >= 10 ? 0 : tiling_of(c); }
 // per-CTA residual partials
 static int max_grid(const hg_ctx* c) { return std::min(c->n_el, 32 * c->n_sm); }
 
@@ -172,7 +170,7 @@ static void run_trace(hg_ctx* c) { HG_DISPATCH_P_EULER(c->P, launch_trace_P, c);
 template <int P, typename real>
 static void ns_dispatch(hg_ctx* c, const NSArgs<real>& a) {
   if constexpr (P < 10) {
-    if (stage_variant(c, c->tiling)) { launch_ns_PV<P, real, 1>(c, a); return; }
+    if (stage_variant(c)) { launch_ns_PV<P, real, 1>(c, a); return; }
   }
   launch_ns_PV<P, real, 0>(c, a);
 }
@@ -194,7 +192,7 @@ static void ns_dispatch(hg_ctx* c, const NSArgs<real>& a) {
   }
 template <int P, typename real>
 static void stage_dispatch(hg_ctx* c, const StageArgs<real>& a) {
-  if (stage_variant(c, c->tiling)) launch_stage_PV<P, real, 1>(c, a);
+  if (stage_variant(c)) launch_stage_PV<P, real, 1>(c, a);
   else launch_stage_PV<P, real, 0>(c, a);
 }
 
@@ -1598,10 +1596,9 @@ extern "C" int hg_set_tiling(hg_ctx* c, int32_t variant) {
 extern "C" int hg_get_tiling(const hg_ctx* c, int32_t out[3]) {
   if (!c || !out) return 1;
   if (is_composite(c)) return hg_get_tiling(c->parts[largest_part(c)], out);
-  const int epb = epb_of(c, c->tiling);
-  out[0] = c->tiling;
-  out[1] = epb;
-  const int v = stage_variant(c, c->tiling);
+  const int v = stage_variant(c);
+  out[0] = tiling_of(c);
+  out[1] = c->ns ? epb_ns_of(c->P, v, in_double(c)) : epb_stage(c->P, v);
   out[2] = c->ns ? ns_threads(c->P, v, in_double(c)) : stage_threads(c->P, v);
   return 0;
 }

@@ -63,7 +63,7 @@ struct hg_ctx {
   void* d_face_metric = nullptr;  // [n_el*4][P][4] Ja/J at the side nodes (curved, gradient faces), context precision
   void* d_GT[2] = {nullptr, nullptr};   // gradient traces [n_el*4][P][2][4] per trace parity (as d_T)
   void* d_dQ = nullptr;           // element gradients [n_el][2][4][NP] (Navier-Stokes)
-  int tiling = 0;                 // elements-per-CTA variant of the stage kernels (hg_autotune / hg_set_tiling)
+  int tiling = -1;                // elements-per-CTA variant set by hg_autotune or hg_set_tiling; -1: by the mesh's size
   bool exact = false;             // some face uses the exact Riemann solver (globally or by zone)
   void* d_FX = nullptr;           // its face fluxes of the current stage [n_el*4][P][4], context precision
   int* d_exact_sides = nullptr;   // the element sides (e*4+s) whose face uses the exact solver
