@@ -84,11 +84,14 @@ struct NSArgs {
   int polls;                // limit of a wait for copies (mbar_wait)
 };
 
-// Elements per group and threads per CTA: variant 0, and variant 1 for small meshes.  At order 5 a double group is
-// half a float one: a CTA's shared memory then lets five reside on an SM instead of two (stage and gradient on the
-// cylinder mesh 58.5 -> 56.4 us, with the jumps indicator 36.3 -> 32.9; in float 33.5 against 34.6).
+// Elements per group and threads per CTA: variant 0, and variant 1 for small meshes.  At orders 3 and 5 a double group
+// is half a float one: a CTA's shared memory then lets twice as many and more reside on an SM (order 5, where both
+// variants then have groups of two: stage and gradient on the cylinder mesh 58.5 -> 56.4 us, with the jumps indicator
+// 36.3 -> 32.9, in float 33.5 against 34.6; order 3, 25,000 elements, an RK3 step: interior penalty 189 -> 172 us, with
+// the modal indicator 234 -> 209 us, which groups of eight ran slower than one node per thread did (220 us); in float the
+// learned indicator's weights weigh more on a smaller CTA: shock 512 x 64 955 against 1050 us).
 __host__ __device__ constexpr int epb_ns(int P, bool dbl) {
-  return P == 2 ? 16 : P <= 4 ? 8 : P == 5 ? 4 : P == 6 ? (dbl ? 2 : 4) : P <= 8 ? 2 : 1;
+  return P == 2 ? 16 : P == 3 ? 8 : P == 4 ? (dbl ? 4 : 8) : P == 5 ? 4 : P == 6 ? (dbl ? 2 : 4) : P <= 8 ? 2 : 1;
 }
 __host__ __device__ constexpr int epb_ns_small(int P) { return P <= 3 ? 4 : P <= 6 ? 2 : 1; }
 __host__ __device__ constexpr int epb_ns_of(int P, int variant, bool dbl) { return variant ? epb_ns_small(P) : epb_ns(P, dbl); }
@@ -179,7 +182,9 @@ struct NSTiles {
   real F[FV ? FV * FS : 4];
   alignas(16) real sens[AV ? T / 32 * sensor_scratch(P) : 4];
   unsigned long long mx[GRAD ? 1 : 4][GRAD ? 1 : T / 32];   // per-warp max |QDot| as bits (NaN above all)
-  static constexpr int REGS = sizeof(real) == 8 ? 128 : 80;
+  // Registers a thread that the launch bounds leave.  Order 4 with the Laplacian dissipation alone spills 250 bytes a
+  // thread at 128 (jumps indicator on 800 curved elements 55.1 -> 45.0 us an RK3 step, 16,000 elements 208 -> 181).
+  static constexpr int REGS = sizeof(real) == 8 ? (P == 5 && IP && AV && !VISC ? 168 : 128) : 80;
   uint64_t bar[2];                     // inputs, RK register
   __device__ __forceinline__ const double* state(int b) const { return KEEP_Q ? in[b].Q : one.Q; }
 };
