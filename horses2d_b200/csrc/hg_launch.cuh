@@ -22,6 +22,18 @@ static int resident_ctas(const hg_ctx* c, std::atomic<int>* known, K kernel, int
   return n;
 }
 
+// CTAs of a persistent launch over `groups` groups of elements, at most `most` resident.  Every CTA takes the same number
+// of groups but the last ones, and there are no more CTAs than that needs.  With few groups to a CTA (`few` or less) that
+// leaves up to half of the residency empty, and an SM a CTA more or less than its neighbour: there all resident CTAs run,
+// some of them for a group more (an RK3 step of 3,750 elements, order 3, interior penalty in double: 41 -> 36 us, 2,400
+// elements of order 4 with BR1 56 -> 51 us).  With many the even split is the faster one (cylinder 64 x 128 N = 5 in
+// double 780 us against 876, shock 512 x 64 1455 against 1555), for Euler from four on: the members of an ensemble run
+// beside one another and fill what each leaves (128 boxes 2.63 against 2.71 ms).
+static inline int persistent_grid(int groups, int most, int few) {
+  const int rounds = (groups + most - 1) / most;
+  return rounds <= few ? std::min(groups, most) : (groups + rounds - 1) / rounds;
+}
+
 // Launch that may overlap the end of the kernel before it on the stream (grid_wait, hg_stage.cuh).  Not under
 // per-kernel timing, whose events stand between the kernels.
 template <typename... KA, typename... A>
@@ -65,8 +77,7 @@ static void launch_stage_PAL(hg_ctx* c, const StageArgs<real>& a) {
   static std::atomic<int> known[HG_KNOWN_DEVICES];
   const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
   const int most = c->n_sm * std::min(32, resident_ctas(c, known, stage_kernel<P, V, real, AFFINE, LGL>, Tl::T, sizeof(Tl), sizeof(Tl)));
-  // every CTA takes the same number of groups but the last ones: no more CTAs than that needs
-  const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
+  const int grid = persistent_grid(groups, most, 3);
   const StageOps<P, real> op = stage_ops<P, real>(c);
   timed(c, HG_KERNEL_STAGE, [&] { launch_dependent(c, stage_kernel<P, V, real, AFFINE, LGL>, grid, Tl::T, sizeof(Tl), a, op); });
   ++c->launches;
@@ -127,7 +138,7 @@ static void launch_groups(hg_ctx* c, std::atomic<int>* known, K kernel, int kind
   const size_t smem = sizeof(Tl) + (weights ? MLP_BYTES : 0);
   const int groups = (a.n_el + Tl::EPB - 1) / Tl::EPB;
   const int most = c->n_sm * std::min(32, resident_ctas(c, known, kernel, Tl::T, smem, sizeof(Tl) + MLP_BYTES));
-  const int rounds = (groups + most - 1) / most, grid = (groups + rounds - 1) / rounds;
+  const int grid = persistent_grid(groups, most, 4);
   timed(c, kind, [&] { launch_dependent(c, kernel, grid, Tl::T, smem, a, op); });
   ++c->launches;
 }
