@@ -219,7 +219,7 @@ static void run_ns_stage(hg_ctx* c, double ca, double cb, double cc, bool first,
   a.GT = static_cast<real*>(c->d_GT[c->cur]);
   a.GT_out = static_cast<real*>(c->d_GT[c->cur ^ 1]);
   a.dQ = static_cast<real*>(c->d_dQ);
-  a.viscous = (c->pc.mu != 0.0 || c->av == HG_AV_PHYSICAL) ? 1 : 0;
+  a.viscous = ns_viscous(c) ? 1 : 0;
   // BR1 always needs the lifted gradient; IP only for gradient traces (viscous fluxes) or the modal and
   // learned indicators on the first stage of a step; the jumps indicator has its own kernel every stage
   a.run_jumps = (c->av != HG_AV_NONE && c->sensor_kind == HG_SENSOR_JUMPS) ? 1 : 0;

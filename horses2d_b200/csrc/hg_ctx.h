@@ -201,6 +201,11 @@ inline bool is_composite(const hg_ctx* c) { return !c->parts.empty(); }
 inline bool ns_fused(const hg_ctx* c) {
   return c->ns && c->ip && !c->is_part && !is_composite(c) && (c->av == HG_AV_NONE || c->sensor_kind != 0);
 }
+// Whether the viscous terms are evaluated.  Without artificial dissipation the stage kernels always do (one instantiation):
+// also where the viscosity is zero, 1 / Re of an infinite Re, so that what they read has been written.
+inline bool ns_viscous(const hg_ctx* c) {
+  return c->ns && (c->pc.mu != 0.0 || c->av != HG_AV_LAPLACIAN);
+}
 constexpr int HG_KNOWN_DEVICES = 16;   // devices whose kernel occupancy is looked up once
 constexpr int HG_MAX_PARTS = 12;
 constexpr int HG_MAX_ORDER_EULER = 12;

@@ -377,7 +377,7 @@ void launch_mortar(hg_ctx* c, int mode) {
     if (mode == MORTAR_FLUX && c->ns && c->ip) mode = MORTAR_FLUX_IP;
     a.mode = mode;
     a.av = c->av;
-    a.visc = c->ns && (c->pc.mu != 0.0 || c->av == HG_AV_PHYSICAL);
+    a.visc = ns_viscous(c);
     a.grad_faces = c->grad_faces ? 1 : 0;
     a.sigma0 = c->sigma0;
     a.epsilon = c->epsilon;

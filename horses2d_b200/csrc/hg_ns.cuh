@@ -58,7 +58,7 @@ struct NSArgs {
   real* GT;                 // dQ traces of the current state [n_el*4][P][2][4]
   real* GT_out;             // dQ traces of the updated state (fused interior-penalty stages)
   real* dQ;                 // element gradients              [n_el][2][4][NP]
-  int viscous;              // viscous fluxes present: mu != 0 or the Physical artificial viscosity
+  int viscous;              // viscous fluxes present (ns_viscous)
   int run_gradient;         // host side: whether this stage needs the gradient kernel
   int run_jumps;            // host side: whether it needs the jumps kernel
   int run_stage;            // host side: whether to launch the stage kernel (a composite runs the
