@@ -126,7 +126,8 @@ static NSOps<P, real> ns_ops(const hg_ctx* c) {
   put(o.hatD, P * P);
   put(o.lb0, P); put(o.lb1, P); put(o.lbw0, P); put(o.lbw1, P);
   put(o.D, P * P);
-  put(o.dlbw0, P); put(o.dlbw1, P); put(o.w, P);
+  put(o.dlbw0, P); put(o.dlbw1, P);
+  m += P;
   put(o.Vinv, P * P);
   return o;
 }
@@ -154,7 +155,8 @@ static void launch_ns_PAI(hg_ctx* c, const NSArgs<real>& a) {
   }
   if (AV && a.run_jumps) {
     EdgeWeights<P, real> ew;
-    for (int k = 0; k < P; ++k) ew.w[k] = op.w[k];
+    const double* w = c->h_mats.data() + 2 * P * P + 6 * P;
+    for (int k = 0; k < P; ++k) ew.w[k] = real(w[k]);
     const int grid = (a.n_el + jumps_epb(P) - 1) / jumps_epb(P);
     timed(c, HG_KERNEL_GRADIENT, [&] { launch_dependent(c, jumps_kernel<P, real, AFFINE>, grid, 128, 0, a, ew); });
     ++c->launches;

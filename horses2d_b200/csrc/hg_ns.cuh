@@ -102,7 +102,7 @@ __host__ __device__ constexpr int ns_threads(int P, int variant, bool dbl) {
 // Nodal operators, passed by value (constant bank); dl = lb^T D, the normal derivatives at the sides.
 template <int P, typename real>
 struct NSOps {
-  real hatD[P * P], D[P * P], lb0[P], lb1[P], lbw0[P], lbw1[P], dlbw0[P], dlbw1[P], dl0[P], dl1[P], w[P], Vinv[P * P];
+  real hatD[P * P], D[P * P], lb0[P], lb1[P], lbw0[P], lbw1[P], dlbw0[P], dlbw1[P], dl0[P], dl1[P], Vinv[P * P];
 };
 
 // out = M in, row by row
@@ -189,7 +189,8 @@ struct NSTiles {
   __device__ __forceinline__ const double* state(int b) const { return KEEP_Q ? in[b].Q : one.Q; }
 };
 // CTAs per SM the launch bounds ask for: what shared memory holds, down to Tl::REGS registers a thread.  Left
-// to itself the compiler takes up to twice as many for the phase with the longest expressions.
+// to itself the compiler takes up to twice as many for the phase with the longest expressions.  (A learned launch holds
+// the network's weights too and may have a CTA less.)
 template <typename Tl>
 constexpr int ns_min_ctas() {
   return cmax(1, cmin(cmin(int(227 * 1024 / (sizeof(Tl) + 1024)), 65536 / (Tl::T * Tl::REGS)), 32));
@@ -453,7 +454,8 @@ template <int P, typename real, bool AFFINE>
 __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSArgs<real> a,
                                                     const __grid_constant__ EdgeWeights<P, real> ew) {
   constexpr int FT = 4 * P, EPB = jumps_epb(P);
-  __shared__ real jr_[EPB * FT], je_[EPB * FT];
+  __shared__ real jr_[EPB * FT], je_[EPB * FT], sr_[EPB * 4], se_[EPB * 4];
+  __shared__ bool rev_[EPB * 4];
   __shared__ real s_w[P];
   const int tid = threadIdx.x, e0 = blockIdx.x * EPB, n_act = min(EPB, a.n_el - e0);
   if (tid < P) {
@@ -464,14 +466,21 @@ __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSAr
   }
   Phys<real> ph;
   ph.load(a.pc);
+  // constant tables, ahead of the wait for the kernel before
+  const int kk = tid % P;
+  const size_t sbase = size_t(e0) * 4 + tid / P, slot = size_t(e0) * FT + tid;
+  const int4 sd = tid < n_act * FT ? a.side[sbase] : make_int4(0, 0, 0, 0);
+  const int kind = sd.y & 15;
+  double visc = 0.0, area = 1.0;
+  if (tid < n_act) {
+    visc = a.av_el[2 * size_t(e0 + tid)];
+    area = a.av_el[2 * size_t(e0 + tid) + 1];
+  }
   __syncthreads();
   grid_wait();
   grid_launch_next();
   if (tid < n_act * FT) {
-    const int sd_ = (tid % FT) / P, kk = tid % P;
-    const size_t sbase = size_t(e0) * 4 + tid / P, slot = size_t(e0) * FT + tid;
-    const int4 sd = a.side[sbase];
-    const int kind = sd.y & 15;
+    if (kk == 0) rev_[tid / P] = kind == SIDE_RIGHT && (sd.y & SIDE_REVERSED);
     if (kind == SIDE_FLUX) {   // edge between orders or subdivided edge: the mortar kernel's jump sums
       jr_[tid] = kk == 0 ? a.NJ[size_t(sd.x) * 2] : real(0);
       je_[tid] = kk == 0 ? a.NJ[size_t(sd.x) * 2 + 1] : real(0);
@@ -499,26 +508,28 @@ __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSAr
       jr_[tid] = s_w[kk] * jr * jr * dSn;
       je_[tid] = s_w[kk] * je * je * dSn;
     }
-    (void)sd_;
+  }
+  __syncthreads();
+  if (tid < n_act * 4) {   // a side's sum, in its edge's order
+    const bool rev = rev_[tid];
+    real sr = real(0), se = real(0);
+    for (int n = 0; n < P; ++n) {
+      const int x = tid * P + (rev ? (P - 1 - n) : n);
+      sr = sr + jr_[x];
+      se = se + je_[x];
+    }
+    sr_[tid] = sr;
+    se_[tid] = se;
   }
   __syncthreads();
   if (tid < n_act) {
-    const int e = e0 + tid;
     real gr = real(0), ge = real(0);
 #pragma unroll
     for (int sd_ = 0; sd_ < 4; ++sd_) {
-      const int fl = a.side[size_t(e) * 4 + sd_].y;
-      const bool rev = (fl & 15) == SIDE_RIGHT && (fl & SIDE_REVERSED);
-      real sr = real(0), se = real(0);
-      for (int n = 0; n < P; ++n) {
-        const int kk = tid * FT + sd_ * P + (rev ? (P - 1 - n) : n);
-        sr = sr + jr_[kk];
-        se = se + je_[kk];
-      }
-      gr = gr + sr;
-      ge = ge + se;
+      gr = gr + sr_[tid * 4 + sd_];
+      ge = ge + se_[tid * 4 + sd_];
     }
-    double gk = double(gr > ge ? gr : ge) / a.av_el[2 * size_t(e) + 1];
+    double gk = double(gr > ge ? gr : ge) / area;
     gk = gk > 1.0e-8 ? log10(gk) : -1.7976931348623157e308;
     const double k = 5.0;
     const double s0 = log10(1.0 / ((P * P) * double(P * P))) + 1.0;
@@ -526,7 +537,7 @@ __global__ void __launch_bounds__(128) jumps_kernel(const __grid_constant__ NSAr
     if (gk < s0 - k) G = 0.0;
     else if (gk < s0 + k) G = 0.5 * sin(0.5 * 3.141592653589793238462643 * (gk - s0) / k) + 0.5;
     else G = 1.0;
-    a.mu_av[e] = a.av_el[2 * size_t(e)] * G;
+    a.mu_av[e0 + tid] = visc * G;
   }
 }
 
