@@ -22,14 +22,16 @@
 //
 // Both kernels are built like the Euler stage kernel (hg_stage.cuh): persistent CTAs over groups of EPB
 // elements with the next group's inputs in flight, and inside a group phases over items (face nodes, volume
-// nodes, lines) between barriers.  Every product with a nodal operator is a line: one thread holds the P
-// nodes of a (variable, line) in registers and takes the operator from the constant bank.  The kernels before
-// held one node per thread and read the operators and the tiles from shared memory, 1.25 loads per
-// multiply-add: their shared-memory pipe ran at 78-81 % of its peak at N = 7 with a quarter of the FP64 rate
-// used, and a third of the warps' time went into global loads at the phase that needed them.  Measured per stage
-// (then -> now): shear layer 384 x 384 N = 7 SIPG FP64 1.57 -> 1.10 ms, FP32 0.81 -> 0.65 ms; cylinder 64 x 128 N = 5
-// BR1 FP64 90 -> 57 us, FP32 54 -> 34 us; shock 512 x 64 N = 3 FP64 62 -> 51 us, FP32 35 -> 32 us.  What bounds them
-// now: the chain of a face task (700 instructions in double) at 12 to 24 warps per SM, and barriers.
+// nodes, lines) between barriers.  A product with a nodal operator is a line: one thread holds the P
+// nodes of a (variable, line) in registers and takes the operator from the constant bank (BR1 in float:
+// row_sums and node_volume_gradient, a node's sums in one order).  The kernels before held one node per
+// thread and read the operators and the tiles from shared memory, 1.25 loads per multiply-add: their
+// shared-memory pipe ran at 78-81 % of its peak at N = 7 with a quarter of the FP64 rate used, and a third
+// of the warps' time went into global loads at the phase that needed them.  Measured per stage (then ->
+// now): shear layer 384 x 384 N = 7 SIPG FP64 1.57 -> 1.04 ms, FP32 0.81 -> 0.62 ms; cylinder 64 x 128 N = 5
+// BR1 (both kernels and the residuals) FP64 89 -> 65 us, FP32 53 -> 42 us; shock 512 x 64 N = 3 FP64
+// 62 -> 48 us, FP32 35 -> 32 us.  What bounds them now: the chain of a face task (700 instructions in
+// double) at 12 to 24 warps per SM, and barriers.
 #pragma once
 #include "hg_stage.cuh"
 #include "hg_sensor.cuh"

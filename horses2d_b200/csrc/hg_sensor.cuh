@@ -2,7 +2,7 @@
 //
 // Three indicators feed the same viscosity law mu_e = Ceps sqrt(Volume)/(N+1) G (the law of
 // JumpsBasedElementViscosity, Approximation/DGArtificialDissipation.f90:322-336):
-//   jumps    the reference's interface-jumps indicator (hg_ns.cuh element_viscosity);
+//   jumps    the reference's interface-jumps indicator (jumps_kernel, hg_ns.cuh);
 //   modal    modal decay (Persson-Peraire): s = max over rho, p of log10(E_N / E), E the energy of
 //            the element's orthonormal-Legendre modal coefficients and E_N that of the modes whose
 //            higher index is N; G = ramp(s; s0, kappa), the same sine ramp as the jumps indicator;

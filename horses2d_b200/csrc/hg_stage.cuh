@@ -21,8 +21,8 @@
 // What bounds it: latency, with 15 warps per SM in double (registers and shared memory), then the shared-memory
 // pipe (58 %); in float instruction issue (70 %).  One thread per node with its loads where they were used (the form
 // before) spent half of its warps' cycles on global loads and filled 62 % of the lanes of its face phase; measured
-// with 512 x 512 elements, N = 4, Gauss-Lobatto, FP64: 0.80 ms a stage then, 0.31 ms now (1.17 GB of state, register
-// and trace traffic: 3.8 TB/s); 16 x 16 elements: 20.5 -> 10.8 us a step.  Fewer or more elements to a group (4, 6)
+// with 512 x 512 elements, N = 4, Gauss-Lobatto, FP64: 0.81 ms a stage then, 0.33 ms now (1.17 GB of state, register
+// and trace traffic: 3.6 TB/s); 16 x 16 elements: 20.5 -> 12.3 us a step.  Fewer or more elements to a group (4, 6)
 // and 96 to 256 threads came out between equal and 25 % slower at N = 4.
 // The Riemann flux of an interior face is evaluated by both of its elements with identical arguments
 // (LEFT trace, RIGHT trace, LEFT's normal), so both see the same value and the face needs no separate
@@ -259,11 +259,12 @@ __host__ __device__ constexpr int face_node(int P, int side, int l, int kk) {
   return (side == 0 || side == 2) ? (l * P + kk) : (kk * P + l);
 }
 
-// In float a node's contraction and lift are one sum in one order: for l = 0 .. N the xi term, then the eta term,
-// then the bottom, right, top and left sides.  A 32-bit time derivative of a smooth state is a difference of sums a
-// thousand times as large, so another order gives it other digits from the fourth on (the two directions summed
-// apart: 3e-4 in the 2-norm at N = 8, against 5e-11 in double, whose kernels do that: one line of one direction per
-// thread).  The lanes of a row of nodes hold different rows j of hatD: a copy in shared memory, transposed.
+// In float (this kernel, and BR1's in hg_ns.cuh) a node's contraction and lift are one sum in one order: for l = 0 .. N
+// the xi term, then the eta term, then the bottom, right, top and left sides.  A 32-bit time derivative of a smooth state
+// is a difference of sums a thousand times as large, so another order gives it other digits from the fourth on (the two
+// directions summed apart: 3e-4 in the 2-norm at N = 8, against 5e-13 in double, whose kernels do that: one line of one
+// direction per thread).  The lanes of a row of nodes hold different rows j of hatD: a copy in shared memory, transposed.
+// Against a line per thread: 128 vortex boxes 2.41 -> 2.54 ms for six steps.
 template <int P, typename real, bool USED = sizeof(real) == 4>
 struct SumOps {
   static constexpr bool ON = USED;
@@ -528,9 +529,9 @@ __global__ void __launch_bounds__(stage_threads(P, V))
     __syncthreads();
 
     // C: time derivative and update, W variables of a node to a lane.  In double two lanes share a node: 16-byte
-    // records side by side over the lanes, in shared memory as in HBM (16 x 16 elements 12.3 -> 10.8 us a step,
-    // orders 5 and 7 with mortars 4.4 -> 4.2 ms; in float, whose records are half as long, a lane per node is the
-    // faster one: 128 vortex boxes 2.44 against 2.66 ms)
+    // records side by side over the lanes, in shared memory as in HBM (16 x 16 elements 12 % less a step, orders 5
+    // and 7 with mortars 5 %; in float, whose records are half as long, a lane per node is the faster one: 128 vortex
+    // boxes 9 %)
     for (int x = tid; x < (4 / W * Tl::NN + 31) / 32 * 32; x += T) {
       const int m = x / (4 / W), h = x % (4 / W) * W;
       const bool on = m < n_act * NP;
