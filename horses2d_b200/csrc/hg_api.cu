@@ -124,9 +124,14 @@ static void health_check(hg_ctx* c) {
 // of latency, and the smaller groups spread it over the chip (an RK3 step at N = 4 in double: 800 elements 15.9 us with
 // variant 0 and 12.8 with variant 1, 16,000 elements 77 and 107).
 static bool in_double(const hg_ctx* c) { return c->precision == HG_PREC_FP64; }
+// From order 8 on variant 1's CTAs of one element (160 to 256 threads) reside two to an SM, from order 11 on one: more
+// elements than that take it a second pass, which variant 0 takes longer to need (order 8, 370 elements 23.1 us with
+// variant 1 and 21.0 with variant 0, 247 elements 15.9 and 19.0; order 12, 177 elements 30.2 and 23.0, 118 elements 18.9
+// and 22.4).
 static int tiling_of(const hg_ctx* c) {
   if (c->tiling >= 0) return c->tiling;
-  return c->n_el < 2 * c->n_sm * (c->ns ? epb_ns_of(c->P, 0, in_double(c)) : epb_stage(c->P, 0)) ? 1 : 0;
+  const int few = c->ns ? 2 * epb_ns_of(c->P, 0, in_double(c)) : c->P >= 12 ? 1 : c->P >= 9 ? 2 : 2 * epb_stage(c->P, 0);
+  return c->n_el < few * c->n_sm ? 1 : 0;
 }
 // The kernels' variant: Navier-Stokes orders 9 and 10 run one element per group in both, one instantiation.
 static int stage_variant(const hg_ctx* c) { return c->ns && c->P >= 10 ? 0 : tiling_of(c); }

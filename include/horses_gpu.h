@@ -275,8 +275,7 @@ const char* hg_group_last_error(const hg_group* group);   /* group may be NULL: 
  * mixed-order meshes -- for each variant in ms_per_variant[HG_TILINGS], both may be NULL), and
  * leaves the residual of the resident state for hg_residuals as hg_time_derivative does; the
  * state is not changed.
- * hg_set_tiling forces a variant (before, the context takes variant 1 on a mesh with fewer than two of variant 0's CTAs
- * per SM, else variant 0); hg_get_tiling: out = {variant in use, elements per CTA, threads
+ * hg_set_tiling forces a variant (before, the context takes variant 1 on a mesh of a few elements per SM, else variant 0); hg_get_tiling: out = {variant in use, elements per CTA, threads
  * per CTA}.  Results are the same in every variant to rounding of the per-CTA reductions. */
 #define HG_TILINGS 2
 int  hg_autotune(hg_ctx* ctx, int32_t trials, int32_t* chosen, double* ms_per_variant);
